@@ -32,6 +32,7 @@
 #include "../../../include/dvmh_gb.h"
 #include "../../../include/dvmh_gb_kernels.h"
 #include "devinfo.cuh"
+#include "fixlimb.cuh"
 #include "softfp64.cuh"
 
 namespace {
@@ -74,6 +75,12 @@ __global__ void __launch_bounds__(UPD_THREADS) kUpdate(double *A, const double *
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint64_t mb = 0, qmax = 0;  // FP64-unit / integer-pipe MAX parts (native == 2: the latter)
     bool seen = false;
+    int E = sf::Q64_E;  // the fixed-point range's smallest exponent field: it follows the values this thread meets
+    auto flush = [&]() {
+        const double d = __ull2double_rn(qmax) * 0x1p-64 * sf::from((uint64_t)(E + 12) << 52);  // RN(max |b - a|)
+        if (sf::bits(d) > mb) mb = sf::bits(d);
+        qmax = 0;
+    };
     const unsigned wstride = gridDim.x * (UPD_THREADS / 32);
     // UNITS units per trip: all their loads are issued before any is used
     constexpr int UNITS = 4;
@@ -101,12 +108,21 @@ __global__ void __launch_bounds__(UPD_THREADS) kUpdate(double *A, const double *
             bool in0 = k0[q] >= lo2 && k0[q] <= hi2, in1 = k0[q] + 1 >= lo2 && k0[q] + 1 <= hi2;
             bool ok = native == 2;
             if (ok) {
-                // |B - A| exact as 64-bit fixed point for values in [2^-12, 1) (see kStencil3)
-                const uint64_t b0 = sf::q64(b[q].x, ok), a0 = sf::q64(a[q].x, ok);
-                const uint64_t b1 = sf::q64(b[q].y, ok), a1 = sf::q64(a[q].y, ok);
+                // |B - A| exact as 64-bit fixed point for +0 and values of twelve binades (see kStencil3), [2^-12, 1) at
+                // first; a pair outside them takes the FP64 unit and moves them to end with its largest value
+                const uint64_t b0 = sf::q64(b[q].x, ok, E), a0 = sf::q64(a[q].x, ok, E);
+                const uint64_t b1 = sf::q64(b[q].y, ok, E), a1 = sf::q64(a[q].y, ok, E);
                 const uint64_t d0 = b0 > a0 ? b0 - a0 : a0 - b0, d1 = b1 > a1 ? b1 - a1 : a1 - b1;
                 if (ok && in0 && d0 > qmax) qmax = d0;  // only exact differences enter the maximum
                 if (ok && in1 && d1 > qmax) qmax = d1;
+                if (!ok) {
+                    const uint32_t top = max(max(sf::hi32(sf::bits(b[q].x)), sf::hi32(sf::bits(a[q].x))),
+                                             max(sf::hi32(sf::bits(b[q].y)), sf::hi32(sf::bits(a[q].y)))) >> 20;
+                    if (top > 64 && top < 2000) {  // no sign bit, and no overflow or underflow of the scaling
+                        flush();
+                        E = (int)top - 11;
+                    }
+                }
             }
             if (!ok) {  // native 0 / 1, or a value outside the fixed-point range (rare)
                 if (in0) mb = sf::absmax_bits(native ? sf::nadd(b[q].x, -a[q].x) : sf::sub(b[q].x, a[q].x), mb);
@@ -118,12 +134,8 @@ __global__ void __launch_bounds__(UPD_THREADS) kUpdate(double *A, const double *
             else if (in1) A[off[q] + 1] = b[q].y;
         }
     }
-    double m = -__builtin_huge_val();
-    if (seen) {
-        const double qd = __ull2double_rn(qmax) * 0x1p-64, f = sf::from(mb);  // RN(max |b - a|), then MAX
-        m = qd > f ? qd : f;
-    }
-    m = ctaMax(m, sh);
+    flush();
+    const double m = ctaMax(seen ? sf::from(mb) : -__builtin_huge_val(), sh);
     if (threadIdx.x == 0) items[blockIdx.x] = m;
 }
 
@@ -802,7 +814,15 @@ __global__ void __launch_bounds__(TX *TY, MINB) kStencil3QF(double *A, const dou
     if (ty == 0 && lane == 0) items[blockIdx.x + gridDim.x * ((long)blockIdx.y + (long)gridDim.y * blockIdx.z)] = m;
 }
 
+struct St3Geom {
+    dim3 grid;
+    long p0;
+    int ichunk;
+    bool ok;
+};
+
 #include "stencil_tma.cuh"
+#include "stencil_limb.cuh"
 
 // CTAs started on each SM (any starting value: only its residue matters); the
 // share of native CTAs is counted per SM, so that every SM runs both kinds at
@@ -833,13 +853,6 @@ __global__ void __launch_bounds__(TX *TY, MINB) kStencil3Q(const double *__restr
     if (nat > 0 && native) planes3<false>(A, Out, b, p0, ichunk, sm);
     else planes3<true>(A, Out, b, p0, ichunk, sm);
 }
-
-struct St3Geom {
-    dim3 grid;
-    long p0;
-    int ichunk;
-    bool ok;
-};
 
 St3Geom st3Geom(const long lo[3], const long hi[3], int TJ) {
     St3Geom g{};
@@ -1031,24 +1044,34 @@ St2Geom st2Geom(const long lo[2], const long hi[2]) {
 
 struct Slabs {
     int n;
-    int rank;
-    long lo[6][3], cnt[6][3];
-    long start[7];
+    long lo[6][3], cnt[6][3];  // axes outermost first; axes the array does not have: 0 and 1
+    long start[7];             // threads before the slab, a multiple of 32
+    int wide[6];               // a warp per row (else a thread per row)
     long st[3];
 };
 
-__global__ void kCopyOutside(const double *__restrict__ src, double *__restrict__ dst, Slabs s) {
-    long total = s.start[s.n];
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
+// One row (fixed outer indices) per warp where rows have at least 32 elements, one per thread where they are shorter
+// (the faces across the innermost axis: one element each).  Bound by latency: 1.6 M elements around a 512^3 box take
+// 5 us; a thread per element with its three 64-bit divisions took 41.
+__global__ void __launch_bounds__(256) kCopyOutside(const double *__restrict__ src, double *__restrict__ dst, Slabs s) {
+    for (long t = blockIdx.x * 256L + threadIdx.x; t < s.start[s.n]; t += gridDim.x * 256L) {
         int q = 0;
         while (t >= s.start[q + 1]) q++;
-        long r = t - s.start[q], off = 0;
-        for (int d = s.rank - 1; d >= 0; d--) {
-            long c = r % s.cnt[q][d];
-            r /= s.cnt[q][d];
-            off += (s.lo[q][d] + c) * s.st[d];
+        const long u = t - s.start[q];
+        const long row = s.wide[q] ? u >> 5 : u;
+        if (row >= s.cnt[q][0] * s.cnt[q][1]) continue;
+        const long c0 = row / s.cnt[q][1], c1 = row - c0 * s.cnt[q][1];
+        const long off = (s.lo[q][0] + c0) * s.st[0] + (s.lo[q][1] + c1) * s.st[1] + s.lo[q][2] * s.st[2];
+        const long step = s.wide[q] ? 32 : 1, n = s.cnt[q][2];
+        long c = s.wide[q] ? u & 31 : 0;
+        for (; c + 7 * step < n; c += 8 * step) {
+            double v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = src[off + (c + e * step) * s.st[2]];
+#pragma unroll
+            for (int e = 0; e < 8; e++) dst[off + (c + e * step) * s.st[2]] = v[e];
         }
-        dst[off] = src[off];
+        for (; c < n; c += step) dst[off + c * s.st[2]] = src[off + c * s.st[2]];
     }
 }
 
@@ -1059,10 +1082,9 @@ __global__ void kCopyOutside(const double *__restrict__ src, double *__restrict_
 // the q61 fixed-point stencil (kStencil3Q) with (CTAs per SM, native CTAs of
 // every den): 14 (4, 0 of 1), 15 (3, 0 of 1), 16 (4, 1 of 2), 17 (4, 1 of 3),
 // 18 (4, 2 of 5), 19 (3, 1 of 2), 20 (4, 1 of 4), 21 (4, 3 of 5); v = 22, 23:
-// the q61 stencil with its planes staged by TMA (kStencil3T), a ring of 6 / 4
-// plane slots, four CTAs per SM; v = 24, 25, 26: ring of 6 with 1, 2, 3 of the
-// 8 warps on the FP64 unit (the fused entry point runs the update and then the
-// stencil into the second buffer for v = 14..26)
+// the stencil on FP32 limbs with its planes staged by TMA (kStencil3L), shapes
+// DVMHGB_LIMB_SHAPES (the fused entry point runs the update and then the stencil
+// into the second buffer for v = 14..26)
 constexpr int V3Q = 14, V3T = 22, V3 = 27;
 int jtOf3(int v) { return (v >= 6 && v < 12) ? 2 : 1; }
 bool isQ3(int v) { return v >= V3Q && v < V3; }
@@ -1081,32 +1103,49 @@ constexpr int V3_OVERLAP = V3 + 1, V3_OVERLAP_Q = V3 + 2, OVL_CHUNKS = 8;
 // four / three CTAs per SM
 constexpr int V3_QF = V3 + 3;
 bool isQF(int v) { return v == V3_QF || v == V3_QF + 1; }
-// ... and the one-pass pair with its planes staged by TMA (kStencil3T<true>),
-// a ring of 5 / 4 planes, four CTAs per SM
+// ... and the one-pass pair with its planes staged by TMA (kStencil3T), a ring
+// of 5 planes, four / three CTAs per SM
 constexpr int V3_TF = V3 + 5;
 bool isTF(int v) { return v == V3_TF || v == V3_TF + 1; }
 
-// the TMA-staged stencil alone (kStencil3T, M = 0) with NS slots and W
-// FP64-unit warps; a launch above 48 KB of shared memory is opted in once per
-// device
-template <int NS, int W>
-int launchT(const CUtensorMap &map, double *A, double *Out, const Box3 &b, const St3Geom &g, cudaStream_t s) {
-    const int smem = tma::smemBytes(false, NS, W > 0);
-    if (smem > 48 * 1024) {
-        static std::atomic<unsigned long long> optedIn{0};
-        const int dev = gbdev::current();
-        if (dev < 0 || dev >= 64) return -1;
-        if (!(optedIn.load() >> dev & 1ull)) {
-            if (cudaFuncSetAttribute(kStencil3T<0, NS, 4, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-                cudaSuccess)
-                return -1;
-            optedIn.fetch_or(1ull << dev);
-        }
-    }
-    kStencil3T<0, NS, 4, W><<<g.grid, dim3(TX, TY), smem, s>>>(map, map, map, A, nullptr, Out, b, g.p0, g.ichunk,
-                                                               nullptr, dvmhgb_status_word(), nullptr, 0);
+// the TMA-staged limb stencil alone (kStencil3L, M = 0): JT rows of j per thread,
+// NS plane slots, registers capped for MINB CTAs per SM
+template <int JT, int NS, int MINB>
+int launchT(const double *A, double *Out, const Box3 &b, const long st[3], const long lo[3], const long hi[3],
+            cudaStream_t s) {
+    const St3Geom g = stLGeom(lo, hi, JT, MINB);
+    const long ext[3] = {b.e0, b.e1, b.e2};
+    CUtensorMap map;
+    if (!g.ok || !encodeMap3(&map, A, ext, st, limb::BX, limb::rowsOf(JT) + 2)) return -1;
+    static std::atomic<int> occ[gbdev::MAX_DEVICES];
+    const int smem = limb::smemBytes(JT, NS);
+    gbdev::residentCtas(occ, kStencil3L<0, JT, NS, MINB>, TX * TY, smem);  // raises the shared-memory limit
+    kStencil3L<0, JT, NS, MINB><<<g.grid, dim3(TX, TY), smem, s>>>(map, Out, b, g.p0, g.ichunk, nullptr,
+                                                                   dvmhgb_status_word(), nullptr);
     return 0;
 }
+
+// the stencil with the next step's update (kStencil3L, M = 3)
+template <int JT, int NS, int MINB>
+int launchSU(const double *A, double *B, double *Aalt, const Box3 &b, const long st[3], const long lo[3],
+             const long hi[3], double *items, cudaStream_t s) {
+    const St3Geom g = stLGeom(lo, hi, JT, MINB);
+    const long ext[3] = {b.e0, b.e1, b.e2};
+    CUtensorMap map;
+    if (!g.ok || !encodeMap3(&map, A, ext, st, limb::BX, limb::rowsOf(JT) + 2)) return -1;
+    static std::atomic<int> occ[gbdev::MAX_DEVICES];
+    const int smem = limb::smemBytes(JT, NS);
+    gbdev::residentCtas(occ, kStencil3L<3, JT, NS, MINB>, TX * TY, smem);  // raises the shared-memory limit
+    kStencil3L<3, JT, NS, MINB><<<g.grid, dim3(TX, TY), smem, s>>>(map, B, b, g.p0, g.ichunk, items,
+                                                                   dvmhgb_status_word(), Aalt);
+    return 0;
+}
+
+// (rows per thread, plane slots, CTAs per SM) of the limb kernels' variants: the stencil's 22 + v (v < 5) and the
+// cross-step pass's v.  At 512^3, us per call (stencil / cross-step pass with the faces' copy): 0: 703 / 777, 1: 620 /
+// 756, 2: 617 / 764, 3 and 5: 612 / 718, 4: 616 / 746.  Two rows a thread take a quarter fewer instructions per cell and
+// hold half the warps; one row at three CTAs is the fastest at 255^3 too (105 / 130), and by more at small sizes.
+#define DVMHGB_LIMB_SHAPES(C) C(0, 1, 5, 4) C(1, 1, 5, 3) C(2, 2, 5, 2) C(3, 1, 6, 3) C(4, 2, 6, 2) C(5, 1, 6, 3)
 
 template <bool FUSED>
 void launch3(int variant, const St3Geom &g, double *A, const double *B, double *Out, const Box3 &b, double *items,
@@ -1167,16 +1206,13 @@ int dvmhgb_jac3d_stencil(const double *A, double *B, const long st[3], const lon
     if (!g.ok || !A || !B || !rows16(st, 3) || !aligned16(A) || !aligned16(B)) return -1;
     Box3 b{st[0], st[1], ext[0], ext[1], ext[2], lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
     if (isT3(native)) {
-        CUtensorMap map;
-        if (!encodeMap3(&map, A, ext, st, tma::BX, tma::BY)) return -1;
-        cudaStream_t s = (cudaStream_t)stream;
-        double *a = (double *)A;
+        int rc = -1;
         switch (native - V3T) {
-#define CT(V, NS, W) \
-    case V: if (launchT<NS, W>(map, a, B, b, g, s) != 0) return -1; break;
-            CT(0, 6, 0) CT(1, 4, 0) CT(2, 6, 1) CT(3, 6, 2) CT(4, 6, 3)
-#undef CT
+#define C(V, JT, NS, MINB) case V: rc = launchT<JT, NS, MINB>(A, B, b, st, lo, hi, (cudaStream_t)stream); break;
+            DVMHGB_LIMB_SHAPES(C)
+#undef C
         }
+        if (rc != 0) return -1;
     } else {
         launch3<false>(native, g, (double *)A, nullptr, B, b, nullptr, (cudaStream_t)stream);
     }
@@ -1294,11 +1330,11 @@ int dvmhgb_jac3d_fused(double *A, const double *B, double *Bnew, const long st[3
         cudaStream_t s = (cudaStream_t)stream;
         int *status = dvmhgb_status_word();
         if (native == V3_TF)
-            kStencil3T<2, 5, 4, 0><<<g.grid, blk, tma::smemBytes(true, 5), s>>>(mapB, mapA, mapT, A, B, Bnew, b, g.p0,
-                                                                                g.ichunk, items, status, nullptr, 0);
+            kStencil3T<5, 4><<<g.grid, blk, tma::smemBytes(5), s>>>(mapB, mapA, mapT, A, B, Bnew, b, g.p0, g.ichunk, items,
+                                                                    status);
         else
-            kStencil3T<2, 5, 3, 0><<<g.grid, blk, tma::smemBytes(true, 5), s>>>(mapB, mapA, mapT, A, B, Bnew, b, g.p0,
-                                                                                g.ichunk, items, status, nullptr, 0);
+            kStencil3T<5, 3><<<g.grid, blk, tma::smemBytes(5), s>>>(mapB, mapA, mapT, A, B, Bnew, b, g.p0, g.ichunk, items,
+                                                                    status);
         dvmhgb_count_launches(1);
         if (cudaGetLastError() != cudaSuccess) return -1;
         return dvmhgb_copy_outside_box(3, B, Bnew, st, ext, lo, hi, stream);
@@ -1330,54 +1366,36 @@ int dvmhgb_jac3d_fused(double *A, const double *B, double *Bnew, const long st[3
 }
 
 long dvmhgb_jac3d_stnupd_items(const long lo[3], const long hi[3], int variant) {
-    if (variant < 0 || variant >= DVMHGB_JAC3D_STNUPD_VARIANTS) return -1;
-    St3Geom g = st3Geom(lo, hi, TY);
+    St3Geom g{};
+    switch (variant) {
+#define C(V, JT, NS, MINB) case V: g = stLGeom(lo, hi, JT, MINB); break;
+        DVMHGB_LIMB_SHAPES(C)
+#undef C
+        default: return -1;
+    }
     return (long)g.grid.x * g.grid.y * g.grid.z;
 }
 
 int dvmhgb_jac3d_stnupd(const double *A, double *Aalt, double *B, const long st[3], const long ext[3],
                         const long lo[3], const long hi[3], double *items, int variant, void *stream) {
     if (variant < 0 || variant >= DVMHGB_JAC3D_STNUPD_VARIANTS) return -1;
-    St3Geom g = st3Geom(lo, hi, TY);
-    if (!g.ok || !A || !Aalt || !B || !items || A == Aalt || A == B || Aalt == B || !rows16(st, 3) ||
-        !aligned16(A) || !aligned16(Aalt) || !aligned16(B))
+    if (!A || !Aalt || !B || !items || A == Aalt || A == B || Aalt == B || !rows16(st, 3) || !aligned16(A) ||
+        !aligned16(Aalt) || !aligned16(B))
         return -1;
     Box3 b{st[0], st[1], ext[0], ext[1], ext[2], lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
-    CUtensorMap map;
-    if (!encodeMap3(&map, A, ext, st, tma::BX, tma::BY)) return -1;
-    cudaStream_t s = (cudaStream_t)stream;
-    double *a = (double *)A;
-    const int smem = tma::smemBytes(false, 6, true);  // above 48 KB: opted in once per device
-    static std::atomic<unsigned long long> optedIn{0};
-    const int dev = gbdev::current();
-    if (dev < 0 || dev >= 64) return -1;
-    if (!(optedIn.load() >> dev & 1ull)) {
-        if (cudaFuncSetAttribute(kStencil3T<3, 6, 4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(kStencil3T<3, 6, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(kStencil3T<3, 6, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-                cudaSuccess)
-            return -1;
-        optedIn.fetch_or(1ull << dev);
+    int rc = -1;
+    switch (variant) {
+#define C(V, JT, NS, MINB) case V: rc = launchSU<JT, NS, MINB>(A, B, Aalt, b, st, lo, hi, items, (cudaStream_t)stream); break;
+        DVMHGB_LIMB_SHAPES(C)
+#undef C
     }
-    int *status = dvmhgb_status_word();
-    const dim3 blk(TX, TY);
-    // (FP64-unit warps, warps with the integer-pipe |B - A|) of each variant
-    static const int wq[DVMHGB_JAC3D_STNUPD_VARIANTS][2] = {{0, 0}, {1, 0}, {2, 0}, {1, 2}, {1, 4}, {2, 3}};
-    const int w = wq[variant][0], qe = wq[variant][1];
-    if (w == 0)
-        kStencil3T<3, 6, 4, 0><<<g.grid, blk, smem, s>>>(map, map, map, a, nullptr, B, b, g.p0, g.ichunk, items, status,
-                                                         Aalt, qe);
-    else if (w == 1)
-        kStencil3T<3, 6, 4, 1><<<g.grid, blk, smem, s>>>(map, map, map, a, nullptr, B, b, g.p0, g.ichunk, items, status,
-                                                         Aalt, qe);
-    else
-        kStencil3T<3, 6, 4, 2><<<g.grid, blk, smem, s>>>(map, map, map, a, nullptr, B, b, g.p0, g.ichunk, items, status,
-                                                         Aalt, qe);
+    if (rc != 0) return -1;
     dvmhgb_count_launches(1);
     if (cudaGetLastError() != cudaSuccess) return -1;
-    return dvmhgb_copy_outside_box(3, A, Aalt, st, ext, lo, hi, stream);  // A's cells outside the box carry over
+    // A's cells outside the box carry over; the kernel has done those of the box's rows in its columns of k
+    const long k0 = lo[2] & ~1L, k1 = k0 + ((hi[2] - k0) / (2 * TX) + 1) * (2 * TX) - 1;
+    const long clo[3] = {lo[0], lo[1], k0}, chi[3] = {hi[0], hi[1], k1 < ext[2] ? k1 : ext[2] - 1};
+    return dvmhgb_copy_outside_box(3, A, Aalt, st, ext, clo, chi, stream);
 }
 
 long dvmhgb_jac2d_update_items(const long lo[2], const long hi[2]) {
@@ -1498,31 +1516,30 @@ int dvmhgb_copy_outside_box(int rank, const double *src, double *dst, const long
                             const long *lo, const long *hi, void *stream) {
     if (rank < 1 || rank > 3) return -1;
     Slabs s{};
-    s.rank = rank;
-    for (int d = 0; d < rank; d++) s.st[d] = st[d];
-    s.start[0] = 0;
+    const int pad = 3 - rank;  // axes the array does not have
+    for (int d = 0; d < 3; d++) s.st[d] = d < pad ? 0 : st[d - pad];
     // slab (d, side): axis d outside [lo_d, hi_d] on one side, axes < d inside, axes > d anything
     for (int d = 0; d < rank; d++)
         for (int side = 0; side < 2; side++) {
-            long a = side == 0 ? 0 : hi[d] + 1, z = side == 0 ? lo[d] - 1 : ext[d] - 1;
+            const long a = side == 0 ? 0 : hi[d] + 1, z = side == 0 ? lo[d] - 1 : ext[d] - 1;
             if (z < a) continue;
-            int q = s.n;
-            long cells = 1;
+            const int q = s.n;
+            bool empty = false;
+            for (int e = 0; e < 3; e++) s.lo[q][e] = 0, s.cnt[q][e] = 1;
             for (int e = 0; e < rank; e++) {
-                long l, h;
-                if (e < d) { l = lo[e]; h = hi[e]; }
-                else if (e == d) { l = a; h = z; }
-                else { l = 0; h = ext[e] - 1; }
-                s.lo[q][e] = l;
-                s.cnt[q][e] = h - l + 1;
-                cells *= h - l + 1;
+                const long l = e < d ? lo[e] : (e == d ? a : 0), h = e < d ? hi[e] : (e == d ? z : ext[e] - 1);
+                s.lo[q][pad + e] = l;
+                s.cnt[q][pad + e] = h - l + 1;
+                empty = empty || h < l;
             }
-            s.start[q + 1] = s.start[q] + cells;
+            if (empty) continue;
+            s.wide[q] = s.cnt[q][2] >= 32;
+            const long rows = s.cnt[q][0] * s.cnt[q][1];
+            s.start[q + 1] = s.start[q] + (s.wide[q] ? rows * 32 : (rows + 31) / 32 * 32);
             s.n++;
         }
     if (s.n == 0) return 0;
-    long total = s.start[s.n];
-    long blocks = (total + 255) / 256;
+    long blocks = (s.start[s.n] + 255) / 256;
     if (blocks > (long)smCount() * 8) blocks = (long)smCount() * 8;
     kCopyOutside<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(src, dst, s);
     dvmhgb_count_launches(1);

@@ -360,13 +360,16 @@ SF_HD double scale_up(double x, int k) {
 }
 
 // x * 2^64 as an exact 64-bit integer for x = +0 or 2^-12 <= x < 1 (such x are
-// multiples of 2^-64 below 1); ok is cleared for any other x (result 0).
-SF_HD uint64_t q64(double x, bool &ok) {
+// multiples of 2^-64 below 1); ok is cleared for any other x (result 0).  With
+// E, the exponent field of the smallest value: x * 2^(1075 - E) for x = +0 or
+// twelve binades, 2^(E-1023) <= x < 2^(E-1011).
+constexpr int Q64_E = 1011;
+SF_HD uint64_t q64(double x, bool &ok, int E = Q64_E) {
     uint64_t X = bits(x);
-    uint32_t e = hi32(X) >> 20;  // the sign bit makes a negative x out of range
-    bool in = e - 1011u <= 11u;
+    uint32_t e = (hi32(X) >> 20) - (uint32_t)E;  // the sign bit makes a negative x out of range
+    bool in = e <= 11u;
     ok &= in | (X == 0);
-    return in ? ((X & MANT) | HID) << (e - 1011u) : 0;
+    return in ? ((X & MANT) | HID) << e : 0;
 }
 
 // ---------------------------------------------------------------- 61-bit fixed point (stencil sums)

@@ -18,15 +18,13 @@
 
 #define R 3
 // default kernel variants, the fastest measured on GB300 at 512^3 (ms per call): the stencil with its planes
-// staged by TMA, sums in q61 fixed point on the integer pipes and 2 of the CTA's 8 warps on the FP64 unit
-// (0.822; the TMA stencil without FP64-unit warps 0.884, the register-staged fixed-point stencil 1.213, all
-// additions on the FP64 unit 1.464)
+// staged by TMA and the sums on FP32 limbs (0.61; in q61 fixed point on the integer pipes, register-staged 1.21, all
+// additions on the FP64 unit 1.46)
 #define DEF_STN 25
-// the pair: the update kernel, then that stencil into the second buffer (1.354 per step; the one-pass TMA pair
-// 1.66, the update and the TMA stencil running at the same time 1.66, the register-staged one-pass pair 2.01)
+// the pair: the update kernel, then that stencil in place
 #define DEF_FUSED 25
 // a step's stencil with the next step's update in one pass (the pairing the runtime forms across steps)
-#define DEF_STNUPD 5  // 2 FP64-unit warps, 3 warps with the integer-pipe |B - A| (1.092 against 1.130 ms for variant 1, same box)
+#define DEF_STNUPD 5  // 0.72 (the q61 pass it replaced: 1.09)
 
 namespace {
 
@@ -35,11 +33,15 @@ namespace {
 // then for stencils: fixed-point sums, FP64-unit additions per cell, rows per
 // thread, CTAs per SM, share of CTAs on the FP64 unit, and for the pair how it
 // runs (0 one pass, 1 update then stencil, 2 the two overlapped in chunks).
-// (the fixed-point feature is 1 for the register-staged kernels and 1 + ring/6
-// for the TMA-staged ones; the share on the FP64 unit is that of CTAs or of
-// warps)
+// (the fixed-point feature is 1 for the register-staged kernels, 1 + ring/6 for the TMA-staged one-pass pair and
+// 2 + ring/6 for the limb kernels)
 constexpr int NDESC = 8;
 constexpr int V_Q = 14, V_T = 22;  // first fixed-point stencil variant, first TMA-staged one
+// the limb kernels' shapes: rows per thread, planes in the ring, CTAs per SM
+void limbDesc(int shape, float *d) {
+    static const int c[6][3] = {{1, 5, 4}, {1, 5, 3}, {2, 5, 2}, {1, 6, 3}, {2, 6, 2}, {1, 6, 3}};
+    d[2] = 2.0f + (float)c[shape][1] / 6.0f, d[3] = 0, d[4] = (float)c[shape][0], d[5] = (float)c[shape][2], d[6] = 0;
+}
 void stencilDesc(int v, float *d) {
     static const int q[8][3] = {{4, 0, 1}, {3, 0, 1}, {4, 1, 2}, {4, 1, 3}, {4, 2, 5}, {3, 1, 2}, {4, 1, 4}, {4, 3, 5}};
     if (v < 12) {
@@ -49,10 +51,8 @@ void stencilDesc(int v, float *d) {
     } else if (v < V_T) {
         const int *c = q[v - V_Q];
         d[2] = 1, d[3] = 5, d[4] = 1, d[5] = (float)c[0], d[6] = (float)c[1] / (float)c[2];
-    } else {  // TMA-staged: ring planes, warps (of 8) on the FP64 unit
-        static const int t[5][2] = {{6, 0}, {4, 0}, {6, 1}, {6, 2}, {6, 3}};
-        const int *c = t[v - V_T];
-        d[2] = 1.0f + (float)c[0] / 6.0f, d[3] = 5, d[4] = 1, d[5] = 4, d[6] = (float)c[1] / 8.0f;
+    } else {
+        limbDesc(v - V_T, d);
     }
 }
 const float *variantDesc(int handler) {
@@ -60,13 +60,10 @@ const float *variantDesc(int handler) {
     static float su[DVMHGB_JAC3D_STNUPD_VARIANTS * NDESC];
     static bool ready = false;
     if (!ready) {
-        static const int wq[DVMHGB_JAC3D_STNUPD_VARIANTS][2] = {{0, 0}, {1, 0}, {2, 0}, {1, 2}, {1, 4}, {2, 3}};
         for (int v = 0; v < DVMHGB_JAC3D_STNUPD_VARIANTS; v++) {  // handler 4: stencil then the next update, one pass
             float *d = su + v * NDESC;
             d[0] = 1, d[1] = 4;
-            stencilDesc(V_T, d);
-            d[6] = (float)wq[v][0] / 8.0f;  // warps on the FP64 unit
-            d[7] = (float)wq[v][1] / 8.0f;  // warps with the integer-pipe |B - A|
+            limbDesc(v, d);
         }
         for (int v = 0; v < 3; v++) upd[v * NDESC] = 1, upd[v * NDESC + 1] = 1, upd[v * NDESC + 2] = (float)v;
         for (int v = 0; v < DVMHGB_JAC3D_VARIANTS; v++) {
@@ -77,9 +74,10 @@ const float *variantDesc(int handler) {
         for (int v = 0; v < DVMHGB_JAC3D_FUSED_VARIANTS; v++) {
             float *d = fus + v * NDESC;
             d[0] = 1, d[1] = 3;
-            if (v >= DVMHGB_JAC3D_FUSED_T) {  // one pass, fixed point, TMA-staged (rings of 5, 4)
-                stencilDesc(V_T, d);
-                d[2] = v == DVMHGB_JAC3D_FUSED_T ? 1.0f + 5.0f / 6.0f : 1.0f + 4.0f / 6.0f;
+            if (v >= DVMHGB_JAC3D_FUSED_T) {  // one pass, fixed point, TMA-staged (4, 3 CTAs per SM)
+                stencilDesc(V_Q, d);
+                d[2] = 1.0f + 5.0f / 6.0f;
+                d[5] = v == DVMHGB_JAC3D_FUSED_T ? 4.0f : 3.0f;
                 d[7] = 0;
                 continue;
             }

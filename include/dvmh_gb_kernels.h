@@ -41,12 +41,13 @@ int dvmhgb_jac3d_update(double *A, const double *B, const long st[3], const long
  * FP64 unit), with a share of the CTAs computing natively so that the FP64
  * unit works beside the integer pipe -- (CTAs per SM, native CTAs of every
  * den): 14 (4, 0/1), 15 (3, 0/1), 16 (4, 1/2), 17 (4, 1/3), 18 (4, 2/5),
- * 19 (3, 1/2), 20 (4, 1/4), 21 (4, 3/5); v = 22, 23: the fixed-point sums
- * with the source planes staged in shared memory by TMA box copies, a ring of
- * 6 / 4 planes per CTA (a copy that does not land within 2 s
- * writes DVMHGB_ERR_TMA_TIMEOUT to dvmhgb_status_word() and the CTA stops);
- * v = 24, 25, 26: ring of 6, with 1, 2, 3 of the CTA's 8 warps computing their
- * cells on the FP64 unit (division by 6 as one multiply and two FMAs);
+ * 19 (3, 1/2), 20 (4, 1/4), 21 (4, 3/5); v = 22..26: the sums on FP32 limbs
+ * (csrc/kernels/fixlimb.cuh) with the source planes staged in shared memory by
+ * TMA box copies (a copy that does not land within 2 s writes
+ * DVMHGB_ERR_TMA_TIMEOUT to dvmhgb_status_word() and the CTA stops); nine
+ * binades of positive values at a time, which follow the field, the rest on the
+ * FP64 unit -- (rows per thread, planes in the ring, CTAs per SM): 22 (1, 5, 4),
+ * 23 (1, 5, 3), 24 (2, 5, 2), 25 (1, 6, 3), 26 (2, 6, 2);
  * -1 for v outside 0..DVMHGB_JAC3D_VARIANTS-1 */
 #define DVMHGB_JAC3D_VARIANTS 27
 #define DVMHGB_ERR_TMA_TIMEOUT 0x544D4101
@@ -83,10 +84,10 @@ long dvmhgb_jac3d_fused_items(const long lo[3], const long hi[3], int native);
  * the new A into Aalt (a second buffer of A's layout, to become A: A is still
  * read while the pass runs; A's cells outside the box are copied over), MAX
  * partials into items (dvmhgb_jac3d_stnupd_items).  24 bytes a cell.  The
- * TMA-staged fixed-point stencil; variants (warps of 8 on the FP64 unit, warps
- * taking |B - A| as exact fixed-point differences on the integer pipe, the
- * rest on the FP64 unit): 0 (0, 0), 1 (1, 0), 2 (2, 0), 3 (1, 2), 4 (1, 4),
- * 5 (2, 3).  The runtime pairs the loops so when a program's time steps leave
+ * limb stencil (variant 25 above) with the update on its new values; variants
+ * (rows per thread, planes in the ring, CTAs per SM): 0 (1, 5, 4), 1 (1, 5, 3),
+ * 2 (2, 5, 2), 3 and 5 (1, 6, 3), 4 (2, 6, 2).
+ * The runtime pairs the loops so when a program's time steps leave
  * the stencil queued past the step's end (deferred loops, dvmh_gb.h). */
 #define DVMHGB_JAC3D_STNUPD_VARIANTS 6
 long dvmhgb_jac3d_stnupd_items(const long lo[3], const long hi[3], int variant);
