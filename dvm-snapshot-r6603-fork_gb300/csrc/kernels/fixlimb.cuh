@@ -262,6 +262,23 @@ SF_HD double assemble(float hm, float mm, float l, float b, int E, int shift = 0
     return sf::from(((uint64_t)res << 32) | lo);
 }
 
+// RN(i u) for an integer |i| < 2^63: normalised to bit 62, its last ten bits rounded to nearest even, +0 for 0
+SF_HD double round63(int64_t i, int E) {
+    const uint32_t sign = (uint32_t)((uint64_t)i >> 32) & 0x80000000u;
+    const uint64_t a = i < 0 ? 0 - (uint64_t)i : (uint64_t)i;
+    const int p = sf::msb32(sf::hi32(a));  // the leading one is bit 32 + p
+    if (p < 0) {                           // below 2^32: exact
+        const uint64_t X = sf::bits((double)i);
+        return sf::from(X == 0 ? 0 : X + ((uint64_t)(int64_t)(E - 1075) << 52));
+    }
+    const uint32_t c = 30u - (uint32_t)p;
+    const uint32_t nh = sf::fshl((uint32_t)a, sf::hi32(a), c), nl = (uint32_t)a << c;
+    const uint64_t n = (((uint64_t)nh << 32) | nl) + (0x1FFu + ((nl >> 10) & 1u));
+    // the significand's leading one adds 1 to the exponent field, a carry out of it 2
+    const uint32_t hi = (sf::hi32(n) >> 10) + ((uint32_t)(p + E - 21) << 20);
+    return sf::from(((uint64_t)(hi | sign) << 32) | sf::fshr((uint32_t)n, sf::hi32(n), 10));
+}
+
 // a double in the range of E (or a sum or quotient of at least 2^52 u) as an integer of u
 SF_HD uint64_t integer(double x, int E) {
     const uint64_t X = sf::bits(x);

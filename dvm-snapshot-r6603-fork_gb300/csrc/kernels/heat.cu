@@ -7,12 +7,33 @@
 // 64-wide chunk of j aligned to a multiple of 64 of the array index (lane l
 // holds j = base+2l, base+2l+1 as one 128-bit access).  Rows i-1, i, i+1 roll
 // through registers with row i+2 in flight, so every source row is read once
-// per chunk; lanes 0 and 31 also fetch the chunk's edge columns.  Per row the
-// warp writes one SUM item -- the pairwise tree over the chunk's 64 positions
-// (pair sum, then xor-butterfly 1..16), the canonical order the reduction
-// engine folds -- and one MINLOC item: the smallest value, ties to the
-// smallest j, i.e. the first in loop order, as the strict '<' of the source
-// gives.  Items are in row-major (row, chunk) order.
+// per chunk; lanes 0 and 31 also fetch the chunk's edge columns.
+//
+// The sum of the four neighbours runs on the FP32 pipe (fixlimb.cuh): a row is
+// split into limbs once, when it arrives, its left and right neighbours come by
+// shuffles of the limbs.  S - 4 src, exact in the limbs' unit, is rounded once
+// from a 63-bit integer, as the source's two operations round it (4 src is exact).
+// The product with c and the last addition are two operations on the FP64 unit.
+// The limbs' range of nine binades follows the values of the warp's rows; a row
+// that does not fit it is computed on the FP64 unit from memory.
+//
+// Per row the warp writes one SUM item -- the pairwise tree over the chunk's 64
+// positions (pair sum, then the lanes by 1, 2, 4, 8, 16), the canonical order
+// the reduction engine folds -- and one MINLOC item: the smallest value, ties to
+// the smallest j, i.e. the first in loop order, as the strict '<' of the source
+// gives.  The pair sums of 8 rows wait in shared memory; then four lanes take a
+// row each and walk its tree in registers: 9 FP64 instructions per 8 rows,
+// where a butterfly per row takes 40.  Items are in row-major (row, chunk) order.
+//
+// What bounds it: about 320 instructions per row of a strip at half the issue
+// rate (16 warps an SM, for 128 registers a thread), and beside them 6.1
+// operations on the FP64 unit, 76 cycles each for a warp.  The kernel that took
+// the sums and the tree's pair on the FP64 unit (13 operations a row) and the
+// rest of the trees as butterflies on the integer pipe: 3171 us for 256 plates of
+// 64..2048 (159 M cells, 380 us of HBM traffic at the copy rate), 124 us for 24
+// of 64..512.  Now 1240 and 25.  On the way: limbs for the four neighbours 1620;
+// S - 4 src on the integer pipe too 1577; the next row's loads no longer waited
+// for in the step that issues them 1240.
 //
 // The same strip code serves one array (plain per-loop launches) and a table
 // of arrays of uneven sizes (batched mode): there the strips of all arrays
@@ -26,6 +47,7 @@
 #include "../../../include/dvmh_gb.h"
 #include "../../../include/dvmh_gb_kernels.h"
 #include "devinfo.cuh"
+#include "fixlimb.cuh"
 #include "softfp64.cuh"
 
 namespace {
@@ -42,112 +64,223 @@ __device__ __forceinline__ uint64_t minKey(double v) {
 
 constexpr int MAX_CACHED = 2048;  // strip bases cached in shared memory
 
-__device__ __forceinline__ double2 ldRow(const double *row, long j, bool need) {
-    return need ? *reinterpret_cast<const double2 *>(row + j) : make_double2(0.0, 0.0);
+constexpr int RB = 8;               // rows whose pair sums wait for their trees, 4 lanes a row
+constexpr int RS = 36;              // stride of such a row: lane l at l + l / 8, read without bank conflicts
+using fx::f32x2;
+
+// a row of the strip: the lane's pair, lane 0's left and lane 31's right edge value, and their limbs
+struct HeatRow {
+    double2 d;
+    double e;
+    fx::Limbs<f32x2> v;
+    float eh, em, el;
+};
+
+// the row's limbs in the range E; false (on every lane) when a lane's values do not fit
+__device__ __forceinline__ bool splitRow(HeatRow &r, int E, bool needY) {
+    if (!needY) r.d.y = r.d.x;  // (not at the load: it would be waited for there)
+    const uint64_t x = sf::bits(r.d.x), y = sf::bits(r.d.y), z = sf::bits(r.e);
+    const uint32_t sx = fx::place(sf::hi32(x), E), sy = fx::place(sf::hi32(y), E), sz = fx::place(sf::hi32(z), E);
+    fx::Raw rx = fx::split(sf::hi32(x), (uint32_t)x, sx), ry = fx::split(sf::hi32(y), (uint32_t)y, sy);
+    fx::Raw rz = fx::split(sf::hi32(z), (uint32_t)z, sz);
+    bool ok = true;
+    if (__any_sync(0xffffffffu, max(max(sx, sy), sz) > 8u)) {
+        rx = fx::splitAny(sf::hi32(x), (uint32_t)x, sx, ok);
+        ry = fx::splitAny(sf::hi32(y), (uint32_t)y, sy, ok);
+        rz = fx::splitAny(sf::hi32(z), (uint32_t)z, sz, ok);
+        ok = __all_sync(0xffffffffu, ok);
+    }
+    r.v = fx::unbias(fx::pack(fx::ffrom(rx.h), fx::ffrom(ry.h)), fx::pack(fx::ffrom(rx.m), fx::ffrom(ry.m)),
+                     fx::pack(fx::ffrom(rx.l), fx::ffrom(ry.l)));
+    r.eh = __fmaf_rn(fx::ffrom(rz.h), 2.0f, -0x1p34f);
+    r.em = fx::ffrom(rz.m) - 0x1p23f;
+    r.el = fx::ffrom(rz.l) - 0x1p23f;
+    return ok;
 }
 
-// strip `local` of loop d: chunk local / nrb, rows (local % nrb) * sr ...
-__device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local) {
+// the limbs' k - 1 and k + 1 neighbours: (left of x, x), (y, right of y)
+__device__ __forceinline__ void sides(f32x2 v, float edge, int lane, f32x2 &left, f32x2 &right) {
+    const float up = __shfl_up_sync(0xffffffffu, fx::hi(v), 1), dn = __shfl_down_sync(0xffffffffu, fx::lo(v), 1);
+    left = fx::pack(lane == 0 ? edge : up, fx::lo(v));
+    right = fx::pack(fx::hi(v), lane == 31 ? edge : dn);
+}
+
+// volatile: the next row's loads stay where they are, a step ahead of their use
+__device__ __forceinline__ double2 ldGlobal2(const double *p) {
+    double2 v;
+    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ldGlobal(const double *p) {
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void stGlobal(double *p, double v) { asm volatile("st.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory"); }
+__device__ __forceinline__ void stGlobal(double *p, double2 v) {
+    asm volatile("st.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ void stGlobal(int *p, int v) { asm volatile("st.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+
+// strip `local` of loop d: chunk local / nrb, rows (local % nrb) * sr ...; sums: RB * RS doubles of the warp's own
+__device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local, double *sums) {
     const int lane = threadIdx.x & 31;
     const long nrows = d.hi0 - d.lo0 + 1;
     const long sr = d.sr;
     const unsigned nrb = (unsigned)((nrows + sr - 1) / sr);
     const unsigned ch = (unsigned)local / nrb, rb = (unsigned)local - ch * nrb;
-    const long r0 = (long)rb * sr, r1 = r0 + sr < nrows ? r0 + sr : nrows;
+    const long r0 = (long)rb * sr;
+    int left = (int)((r0 + sr < nrows ? r0 + sr : nrows) - r0);  // rows to do
     const long base = (d.c0 + ch) * 64;
     const long j = base + 2 * lane;
-    const bool need = j <= d.hi1 + 1;  // the pair holds a cell of the loop or its right neighbour
+    const long last = d.hi1 + 1;  // the last column a cell of the loop reads
     const bool in0 = j >= d.lo1 && j <= d.hi1, in1 = j + 1 >= d.lo1 && j + 1 <= d.hi1;
-    // edge columns: lane 0 the left neighbour of j = base, lane 31 the right one of base + 63
-    const long ej = lane == 0 ? j - 1 : j + 2;
-    const bool eNeed = (lane == 0 && j >= 1) || (lane == 31 && j + 2 <= d.hi1 + 1);
-    const double c = *d.coef;
+    // edge columns: lane 0 the left neighbour of j = base, lane 31 the right one of base + 63.  Elements that no cell of
+    // the loop needs are replaced by others of the row, so that they do not leave the limbs' range.
+    const int jo = j <= last ? 0 : (int)((last & ~1L) - j);                 // the pair's offset from j
+    const bool needY = j + jo + 1 <= last;                                  // its second element (else the row's padding)
+    const int eo = lane == 0 ? (j >= 1 ? -1 : 0) : (lane == 31 && j + 2 <= last ? 2 : jo);
+    const double c = __ldg(d.coef);
     const long s0 = d.s0;
-    const double *p = d.src + (d.lo0 + r0 - 1) * s0;  // row i-1 of the first row
-    double2 up = ldRow(p, j, need), mid = ldRow(p + s0, j, need), dn = ldRow(p + 2 * s0, j, need);
-    double emid = eNeed ? p[s0 + ej] : 0.0, edn = eNeed ? p[2 * s0 + ej] : 0.0;
-    for (long r = r0; r < r1; r++) {
-        const long i = d.lo0 + r;
-        const double *pn = d.src + (i + 2) * s0;  // row i+2, in flight (exists while r + 1 < r1)
-        const bool more = r + 1 < r1;
-        const double2 dn2 = ldRow(pn, j, need && more);
-        const double edn2 = (eNeed && more) ? pn[ej] : 0.0;
-        double left = __shfl_up_sync(0xffffffffu, mid.y, 1), right = __shfl_down_sync(0xffffffffu, mid.x, 1);
-        if (lane == 0) left = emid;
-        if (lane == 31) right = emid;
-        // 4.0 * mid is exact: an exponent increment on the integer pipe unless a
-        // lane of the warp holds a subnormal, infinite or huge value
-        double m4x, m4y;
-        if (__all_sync(0xffffffffu, sf::scale_up_ok(mid.x, 2) && sf::scale_up_ok(mid.y, 2))) {
-            m4x = sf::scale_up(mid.x, 2);
-            m4y = sf::scale_up(mid.y, 2);
-        } else {
-            m4x = 4.0 * mid.x;
-            m4y = 4.0 * mid.y;
-        }
-        const double v0 = mid.x + c * ((((up.x + dn.x) + left) + mid.y) - m4x);
-        const double v1 = mid.y + c * ((((up.y + dn.y) + mid.x) + right) - m4y);
-        double *out = d.dst + i * s0 + j;
-        if (in0 && in1) *reinterpret_cast<double2 *>(out) = make_double2(v0, v1);
-        else if (in0) out[0] = v0;
-        else if (in1) out[1] = v1;
-        // SUM: pairwise tree over the chunk's positions, -0.0 outside the loop.
-        // When every value of the chunk is +0 or a positive normal below 2^1009
-        // the levels above the pairs run on the integer pipe (sf::add_pos); the
-        // positions outside the loop then count as +0, which gives the same
-        // sum, since the chunk has a cell of the loop and no sum is negative.
-        double s;
-        if (__all_sync(0xffffffffu, (!in0 || sf::pos_small(v0)) && (!in1 || sf::pos_small(v1)))) {
-            s = (in0 ? v0 : 0.0) + (in1 ? v1 : 0.0);
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) s = sf::add_pos(s, __shfl_xor_sync(0xffffffffu, s, o));
-        } else {
-            s = (in0 ? v0 : -0.0) + (in1 ? v1 : -0.0);
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o);
-        }
-        // MINLOC: smallest key, then smallest j; the value comes from the winning lane
-        const uint64_t k0 = in0 ? minKey(v0) : ~0ull, k1 = in1 ? minKey(v1) : ~0ull;
-        uint64_t key = k1 < k0 ? k1 : k0;
-        int jo = 2 * lane + (k1 < k0 ? 1 : 0);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const uint64_t ok = __shfl_down_sync(0xffffffffu, key, o);
-            const int oj = __shfl_down_sync(0xffffffffu, jo, o);
-            if (ok < key || (ok == key && oj < jo)) {
-                key = ok;
-                jo = oj;
+    const int nck = (int)d.nck;
+    const double *p = d.src + (d.lo0 + r0 - 1) * s0 + j;  // the pair of row i-1 (+ jo)
+    const long toOut = d.dst - d.src + s0;                // from there to row i of dst
+    int item = (int)(r0 * nck + ch);                      // (a loop's items are fewer than 2^31)
+    int row = (int)(d.lo0 + r0);  // i
+    double *const sumItems = d.sumItems, *const minItems = d.minItems;
+    int *const locItems = d.locItems;
+    int E = fx::E_DEFAULT;
+    auto load = [&](const double *q, HeatRow &r) {
+        r.d = ldGlobal2(q + jo);
+        r.e = ldGlobal(q + eo);
+    };
+    HeatRow ra, rc, rd;
+    load(p, ra);
+    load(p + s0, rc);
+    load(p + 2 * s0, rd);
+    bool okA = splitRow(ra, E, needY), okC = splitRow(rc, E, needY), okD = splitRow(rd, E, needY);
+    int rr = 0;  // rows in the batch
+
+    // row i from up, mid, dn; up then takes row i + 2's place
+    auto step = [&](HeatRow &up, HeatRow &mid, HeatRow &dn, bool &okU, bool &okM, bool &okD) -> bool {
+        HeatRow nx;
+        const bool more = left > 1;
+        if (more) load(p + 3 * s0, nx);
+        if (__builtin_expect(!(okU && okM && okD), 0)) {  // move the range to end with the three rows' largest value
+            load(p, up);
+            load(p + s0, mid);
+            load(p + 2 * s0, dn);
+            const auto top = [](const HeatRow &h) {
+                return max(max(sf::hi32(sf::bits(h.d.x)), sf::hi32(sf::bits(h.d.y))), sf::hi32(sf::bits(h.e)));
+            };
+            const int e = (int)(__reduce_max_sync(0xffffffffu, max(max(top(up), top(mid)), top(dn))) >> 20) - 8;
+            if (e != E && e >= fx::E_MIN && e <= fx::E_MAX) {
+                E = e;
+                okU = splitRow(up, E, needY);
+                okM = splitRow(mid, E, needY);
+                okD = splitRow(dn, E, needY);
             }
         }
-        jo = __shfl_sync(0xffffffffu, jo, 0);
-        const double mine = (jo & 1) ? v1 : v0;
-        const double val = __shfl_sync(0xffffffffu, mine, jo >> 1);
-        if (lane == 0) {
-            const long item = r * d.nck + ch;
-            d.sumItems[item] = s;
-            d.minItems[item] = key == ~0ull ? __builtin_huge_val() : val;
-            d.locItems[2 * item] = (int)i;
-            d.locItems[2 * item + 1] = (int)(base + jo);
+        double v0, v1;
+        if (__builtin_expect(okU && okM && okD, 1)) {
+            fx::Limbs<f32x2> lt, rt;
+            sides(mid.v.h, mid.eh, lane, lt.h, rt.h);
+            sides(mid.v.m, mid.em, lane, lt.m, rt.m);
+            sides(mid.v.l, mid.el, lane, lt.l, rt.l);
+            // ((src[i-1] + src[i+1]) + src[j-1]) + src[j+1]
+            const fx::Limbs<f32x2> s = fx::add(fx::add(fx::add(up.v, dn.v), lt), rt);
+            // S - 4 src as an integer of the limbs' unit, rounded once
+            const f32x2 m4 = fx::pack(-4.0f, -4.0f), sc = fx::pack(0x1p-11f, 0x1p-11f);
+            const f32x2 th = fx::vmul(fx::vfma(mid.v.h, m4, s.h), sc), tm = fx::vfma(mid.v.m, m4, s.m);
+            const f32x2 tl = fx::vfma(mid.v.l, m4, s.l);
+            const int64_t tx = ((int64_t)__float2int_rz(fx::lo(th)) << 40) + ((int64_t)__float2int_rz(fx::lo(tm)) << 20) +
+                               (int64_t)__float2int_rz(fx::lo(tl));
+            const int64_t ty = ((int64_t)__float2int_rz(fx::hi(th)) << 40) + ((int64_t)__float2int_rz(fx::hi(tm)) << 20) +
+                               (int64_t)__float2int_rz(fx::hi(tl));
+            v0 = mid.d.x + c * fx::round63(tx, E);
+            v1 = mid.d.y + c * fx::round63(ty, E);
+        } else {
+            const double *q = p;  // row i-1
+            v0 = v1 = 0.0;
+            if (in0) v0 = q[s0] + c * ((((q[0] + q[2 * s0]) + q[s0 - 1]) + q[s0 + 1]) - 4.0 * q[s0]);
+            if (in1) v1 = q[s0 + 1] + c * ((((q[1] + q[2 * s0 + 1]) + q[s0]) + q[s0 + 2]) - 4.0 * q[s0 + 1]);
         }
-        up = mid;
-        mid = dn;
-        dn = dn2;
-        emid = edn;
-        edn = edn2;
+        double *out = const_cast<double *>(p) + toOut;
+        if (in0 && in1) stGlobal(out, make_double2(v0, v1));
+        else if (in0) stGlobal(out, v0);
+        else if (in1) stGlobal(out + 1, v1);
+        // SUM: -0.0 outside the loop
+        sums[rr * RS + lane + (lane >> 3)] = (in0 ? v0 : -0.0) + (in1 ? v1 : -0.0);
+        // MINLOC: the smallest value's first cell.  Non-negative values below infinity are ordered as their bits are;
+        // other rows go by minKey.  The lane that holds the minimum writes the item.
+        {
+            uint32_t h0 = in0 ? sf::hi32(sf::bits(v0)) : 0x7FF00000u, h1 = in1 ? sf::hi32(sf::bits(v1)) : 0x7FF00000u;
+            uint32_t l0 = (uint32_t)sf::bits(v0), l1 = (uint32_t)sf::bits(v1);
+            bool none = false;  // no cell below infinity
+            if (__builtin_expect(__any_sync(0xffffffffu, max(h0, h1) > 0x7FF00000u || (in0 && h0 == 0x7FF00000u) ||
+                                                             (in1 && h1 == 0x7FF00000u)), 0)) {
+                const uint64_t k0 = in0 ? minKey(v0) : ~0ull, k1 = in1 ? minKey(v1) : ~0ull;
+                h0 = sf::hi32(k0), l0 = (uint32_t)k0, h1 = sf::hi32(k1), l1 = (uint32_t)k1;
+                none = __all_sync(0xffffffffu, (k0 & k1) == ~0ull);
+            }
+            const bool second = h1 < h0 || (h1 == h0 && l1 < l0);
+            const uint32_t h = second ? h1 : h0, l = second ? l1 : l0, mh = __reduce_min_sync(0xffffffffu, h);
+            unsigned who = __ballot_sync(0xffffffffu, h == mh);
+            if (who & (who - 1)) {  // equal high words
+                const uint32_t ml = __reduce_min_sync(0xffffffffu, h == mh ? l : ~0u);
+                who = __ballot_sync(0xffffffffu, h == mh && l == ml);
+            }
+            if (lane == __ffs(who) - 1) {
+                stGlobal(minItems + item, none ? __builtin_huge_val() : second ? v1 : v0);
+                stGlobal(locItems + 2 * (long)item, row);
+                stGlobal(locItems + 2 * (long)item + 1, (int)j + (second ? 1 : 0));
+            }
+        }
+        if (++rr == RB || !more) {
+            __syncwarp();
+            double x[RB];
+            const double *q = sums + (lane >> 2) * RS + (lane & 3) * 9;
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[i] = q[i];
+#pragma unroll
+            for (int w = 1; w < 8; w <<= 1)
+#pragma unroll
+                for (int i = 0; i < 8; i += 2 * w) x[i] = x[i] + x[i + w];
+            double total = x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
+            total = total + __shfl_xor_sync(0xffffffffu, total, 2);
+            if ((lane & 3) == 0 && (lane >> 2) < rr) stGlobal(sumItems + item + ((lane >> 2) + 1 - rr) * nck, total);
+            __syncwarp();
+            rr = 0;
+        }
+        if (!more) return false;
+        up = nx;
+        okU = splitRow(up, E, needY);
+        p += s0;
+        item += nck;
+        row++;
+        left--;
+        return true;
+    };
+    // three rows a trip, so that the limbs stay where they are
+    while (step(ra, rc, rd, okA, okC, okD) && step(rc, rd, ra, okC, okD, okA) && step(rd, ra, rc, okD, okA, okC)) {
     }
 }
 
-__global__ void __launch_bounds__(HT) kHeatOne(dvmhgb_heat_desc d) {
+constexpr int HB = 2;  // CTAs per SM
+
+__global__ void __launch_bounds__(HT, HB) kHeatOne(dvmhgb_heat_desc d) {
+    __shared__ double sums[HT / 32][RB * RS];
     for (long s = (blockIdx.x * (long)HT + threadIdx.x) >> 5; s < d.strips; s += (long)gridDim.x * (HT / 32))
-        heatStrip(d, s);
+        heatStrip(d, s, sums[threadIdx.x >> 5]);
 }
 
 // strips of array k are [d[k].stripBase, d[k].stripBase + d[k].strips)
-__global__ void __launch_bounds__(HT) kHeatMany(const dvmhgb_heat_desc *__restrict__ ds, int n, long total) {
-    __shared__ long sb[MAX_CACHED];
-    const bool cached = n <= MAX_CACHED;
+__global__ void __launch_bounds__(HT, HB) kHeatMany(const dvmhgb_heat_desc *__restrict__ ds, int n, long total) {
+    __shared__ int sb[MAX_CACHED];
+    __shared__ double sums[HT / 32][RB * RS];
+    const bool cached = n <= MAX_CACHED && total < (1L << 31);
     if (cached)
-        for (int q = threadIdx.x; q < n; q += HT) sb[q] = ds[q].stripBase;
+        for (int q = threadIdx.x; q < n; q += HT) sb[q] = (int)ds[q].stripBase;
     __syncthreads();
     for (long s = (blockIdx.x * (long)HT + threadIdx.x) >> 5; s < total; s += (long)gridDim.x * (HT / 32)) {
         int lo = 0, hi = n - 1;  // last array whose stripBase <= s
@@ -156,11 +289,20 @@ __global__ void __launch_bounds__(HT) kHeatMany(const dvmhgb_heat_desc *__restri
             if ((cached ? sb[mid] : ds[mid].stripBase) <= s) lo = mid;
             else hi = mid - 1;
         }
-        heatStrip(ds[lo], s - (cached ? sb[lo] : ds[lo].stripBase));
+        heatStrip(ds[lo], s - (cached ? sb[lo] : ds[lo].stripBase), sums[threadIdx.x >> 5]);
     }
 }
 
-int smCount() { return gbdev::smCount(); }
+long residentWarps() { return (long)gbdev::smCount() * HB * (HT / 32); }
+
+// strips of sr rows over a loop
+long stripsOf(const dvmhgb_heat_desc &d, long sr) { return d.nck * ((d.hi0 - d.lo0 + sr) / sr); }
+
+// What `strips` strips of sr rows cost, in rows of one warp: each begins with three rows loaded and split before its
+// first result, and the warps the GPU holds take them in rounds.  Measured, us: 256 plates of 64..2048 (159 M cells)
+// 1283 / 1241 / 1240 / 1282 at 16 / 32 / 64 / 128 rows; 24 of 64..512 27.7 / 24.8 / 34.9 / 61.7 at 8 / 16 / 32 / 64;
+// 60 of 16..256 14.6 / 20.1 / 33.5 at 8 / 16 / 32.
+long stripCost(long strips, long sr) { return (strips + residentWarps() - 1) / residentWarps() * (2 * sr + 5); }
 
 }  // namespace
 
@@ -195,14 +337,12 @@ int dvmhgb_heat_desc_fill(dvmhgb_heat_desc *d, const double *src, double *dst, l
 
 int dvmhgb_heat(const dvmhgb_heat_desc *d, void *stream) {
     if (!d || !d->sumItems || !d->minItems || !d->locItems) return -1;
-    // one loop alone: strips short enough that there is one for every warp the GPU holds
     dvmhgb_heat_desc e = *d;
-    const long nrows = e.hi0 - e.lo0 + 1, warps = (long)smCount() * 8 * (HT / 32);
-    long sr = (nrows * e.nck + warps - 1) / warps;
-    e.sr = sr < 1 ? 1 : (sr > DVMHGB_HEAT_STRIP ? DVMHGB_HEAT_STRIP : sr);
-    e.strips = e.nck * ((nrows + e.sr - 1) / e.sr);
+    for (long sr = e.sr = 1; sr <= DVMHGB_HEAT_STRIP; sr *= 2)
+        if (stripCost(stripsOf(*d, sr), sr) <= stripCost(stripsOf(*d, e.sr), e.sr)) e.sr = sr;
+    e.strips = stripsOf(e, e.sr);
     long blocks = (e.strips + HT / 32 - 1) / (HT / 32);
-    if (blocks > (long)smCount() * 8) blocks = (long)smCount() * 8;
+    if (blocks > (long)gbdev::smCount() * HB) blocks = (long)gbdev::smCount() * HB;
     kHeatOne<<<(unsigned)blocks, HT, 0, (cudaStream_t)stream>>>(e);
     dvmhgb_count_launches(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -211,14 +351,30 @@ int dvmhgb_heat(const dvmhgb_heat_desc *d, void *stream) {
 int dvmhgb_heat_desc_rows(dvmhgb_heat_desc *d, long sr) {
     if (!d || sr < 1) return -1;
     d->sr = sr;
-    d->strips = d->nck * ((d->hi0 - d->lo0 + sr) / sr);
+    d->strips = stripsOf(*d, sr);
     return d->strips < (1L << 31) ? 0 : -1;
+}
+
+int dvmhgb_heat_default_variant(const dvmhgb_heat_desc *d, int n) {
+    if (!d || n < 1) return -1;
+    int best = -1;
+    long bestCost = 0;
+    for (int v = 0; v < DVMHGB_HEAT_VARIANTS; v++) {
+        if (DVMHGB_HEAT_CTAS(v) != HB) continue;
+        const long sr = DVMHGB_HEAT_ROWS(v);
+        long strips = 0;
+        for (int q = 0; q < n; q++) strips += stripsOf(d[q], sr);
+        const long cost = stripCost(strips, sr);
+        if (best < 0 || cost < bestCost) best = v, bestCost = cost;
+    }
+    return best;
 }
 
 int dvmhgb_heat_many_grid(const dvmhgb_heat_desc *dDev, int n, long totalStrips, int ctasPerSm, void *stream) {
     if (!dDev || n < 1 || totalStrips < 1 || ctasPerSm < 1 || ctasPerSm > 8) return -1;
     long blocks = (totalStrips + HT / 32 - 1) / (HT / 32);
-    if (blocks > (long)smCount() * ctasPerSm) blocks = (long)smCount() * ctasPerSm;
+    if (ctasPerSm > HB) ctasPerSm = HB;  // more would wait for the resident ones' whole walk
+    if (blocks > (long)gbdev::smCount() * ctasPerSm) blocks = (long)gbdev::smCount() * ctasPerSm;
     kHeatMany<<<(unsigned)blocks, HT, 0, (cudaStream_t)stream>>>(dDev, n, totalStrips);
     dvmhgb_count_launches(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

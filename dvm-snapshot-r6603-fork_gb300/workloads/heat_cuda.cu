@@ -27,7 +27,7 @@ void heatVariantDesc(float *d, long loops, long cells, long maxRows) {
     for (int v = 0; v < DVMHGB_HEAT_VARIANTS; v++) {
         float *e = d + v * HEAT_NDESC;
         e[0] = 4;
-        e[1] = (float)(4 + v % 5);
+        e[1] = (float)(3 + v % 5);
         e[2] = (float)DVMHGB_HEAT_CTAS(v);
         e[3] = (float)log2((double)loops);
         e[4] = (float)log2((double)(cells > 1 ? cells : 1));
@@ -100,7 +100,8 @@ extern "C" void loop_heat_batch_cuda(DvmType *refs, DvmType count) {
     }
     float desc[DVMHGB_HEAT_VARIANTS * HEAT_NDESC];
     heatVariantDesc(desc, (long)count, cells, maxRows);
-    const int v = dvmhgb_loop_variant_desc(refs[0], DVMHGB_HEAT_VARIANTS, DVMHGB_HEAT_DEFAULT, desc, HEAT_NDESC);
+    const int dflt = dvmhgb_heat_default_variant(table, (int)count);
+    const int v = dvmhgb_loop_variant_desc(refs[0], DVMHGB_HEAT_VARIANTS, dflt < 0 ? 0 : dflt, desc, HEAT_NDESC);
     long total = 0, units = 0;
     for (DvmType q = 0; q < count; q++) {
         dvmhgb_heat_desc_rows(&table[q], DVMHGB_HEAT_ROWS(v));

@@ -163,12 +163,15 @@ int dvmhgb_heat_many(const dvmhgb_heat_desc *dDev, int n, long totalStrips, void
 /* The strip geometry of the batched step, a tuner choice (results do not depend
  * on it: a strip's SUM and MINLOC items are per (row, chunk) whatever the
  * strip): variant v walks strips of DVMHGB_HEAT_ROWS(v) rows with a persistent
- * grid of DVMHGB_HEAT_CTAS(v) CTAs of 8 warps per SM.  dvmhgb_heat_desc_rows
- * sets a descriptor's rows per strip (and its strip count); -1 for sr < 1. */
+ * grid of DVMHGB_HEAT_CTAS(v) CTAs of 8 warps per SM (the most an SM holds: 2).
+ * dvmhgb_heat_default_variant: the one that costs least for a host table of n
+ * filled descriptors, by the rounds of strips the GPU's warps take (-1 for bad
+ * arguments).  dvmhgb_heat_desc_rows sets a descriptor's rows per strip (and its
+ * strip count); -1 for sr < 1. */
 #define DVMHGB_HEAT_VARIANTS 10
-#define DVMHGB_HEAT_DEFAULT 2
-#define DVMHGB_HEAT_ROWS(v) (16L << ((v) % 5))
-#define DVMHGB_HEAT_CTAS(v) ((v) < 5 ? 8 : 4)
+#define DVMHGB_HEAT_ROWS(v) (8L << ((v) % 5))
+#define DVMHGB_HEAT_CTAS(v) ((v) < 5 ? 2 : 1)
+int dvmhgb_heat_default_variant(const dvmhgb_heat_desc *d, int n);
 int dvmhgb_heat_desc_rows(dvmhgb_heat_desc *d, long sr);
 int dvmhgb_heat_many_grid(const dvmhgb_heat_desc *dDev, int n, long totalStrips, int ctasPerSm, void *stream);
 

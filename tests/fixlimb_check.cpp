@@ -92,3 +92,23 @@ extern "C" long fixlimb_check_range(void) {
     }
     return bad;
 }
+
+// round63 against the FPU's rounding: integers of every length, ties and carries among them
+extern "C" long fixlimb_check_round63(long n, uint64_t seed) {
+    long bad = 0;
+    for (long i = 0; i < n; i++) {
+        const uint64_t r = mix(seed + 2 * (uint64_t)i), q = mix(seed + 2 * (uint64_t)i + 1);
+        uint64_t a = (r | (1ull << 63)) >> (1 + q % 63);
+        switch ((q >> 8) % 4) {
+            case 0: a &= ~((1ull << ((q >> 16) % 60)) - 1); break;
+            case 1: a |= (1ull << ((q >> 16) % 60)) - 1; break;
+            case 2: a = (a & ~1023ull) | 512u | (a >> 12 & 1u); break;  // at and beside the tie of a full-length integer
+            default: break;
+        }
+        a &= (1ull << 63) - 1;
+        const int64_t v = (q >> 32) & 1 ? -(int64_t)a : (int64_t)a;
+        const int E = fx::E_MIN + (int)((q >> 40) % (fx::E_MAX - fx::E_MIN + 1));
+        bad += !same(fx::round63(v, E), std::ldexp((double)v, E - 1075));
+    }
+    return bad + !same(fx::round63(0, fx::E_DEFAULT), 0.0);
+}

@@ -15,8 +15,9 @@ def hostlib(tmp_path_factory):
     subprocess.check_call(["g++", "-O2", "-ffp-contract=off", "-frounding-math", "-std=c++17", "-fPIC", "-shared",
                            os.path.join(HERE, "fixlimb_check.cpp"), "-o", out])
     L = ctypes.CDLL(out)
-    L.fixlimb_check.restype = L.fixlimb_check_range.restype = ctypes.c_long
-    L.fixlimb_check.argtypes = [ctypes.c_long, ctypes.c_uint64]
+    for f in (L.fixlimb_check, L.fixlimb_check_range, L.fixlimb_check_round63):
+        f.restype = ctypes.c_long
+    L.fixlimb_check.argtypes = L.fixlimb_check_round63.argtypes = [ctypes.c_long, ctypes.c_uint64]
     return L
 
 
@@ -27,3 +28,9 @@ def test_sums_and_quotients_match_the_host_fpu(hostlib, seed):
 
 def test_splitting_refuses_what_the_limbs_cannot_hold(hostlib):
     assert hostlib.fixlimb_check_range() == 0
+
+
+@pytest.mark.parametrize("seed", [2, 20261207])
+def test_rounding_of_integers_matches_the_host_fpu(hostlib, seed):
+    """The heat kernel's S - 4 src: a signed 63-bit integer rounded once to a double."""
+    assert hostlib.fixlimb_check_round63(4_000_000, seed) == 0
