@@ -47,8 +47,7 @@
 #include "../../../include/dvmh_gb.h"
 #include "../../../include/dvmh_gb_kernels.h"
 #include "devinfo.cuh"
-#include "fixlimb.cuh"
-#include "softfp64.cuh"
+#include "rowlimb.cuh"
 
 namespace {
 
@@ -67,60 +66,6 @@ constexpr int MAX_CACHED = 2048;  // strip bases cached in shared memory
 constexpr int RB = 8;               // rows whose pair sums wait for their trees, 4 lanes a row
 constexpr int RS = 36;              // stride of such a row: lane l at l + l / 8, read without bank conflicts
 using fx::f32x2;
-
-// a row of the strip: the lane's pair, lane 0's left and lane 31's right edge value, and their limbs
-struct HeatRow {
-    double2 d;
-    double e;
-    fx::Limbs<f32x2> v;
-    float eh, em, el;
-};
-
-// the row's limbs in the range E; false (on every lane) when a lane's values do not fit
-__device__ __forceinline__ bool splitRow(HeatRow &r, int E, bool needY) {
-    if (!needY) r.d.y = r.d.x;  // (not at the load: it would be waited for there)
-    const uint64_t x = sf::bits(r.d.x), y = sf::bits(r.d.y), z = sf::bits(r.e);
-    const uint32_t sx = fx::place(sf::hi32(x), E), sy = fx::place(sf::hi32(y), E), sz = fx::place(sf::hi32(z), E);
-    fx::Raw rx = fx::split(sf::hi32(x), (uint32_t)x, sx), ry = fx::split(sf::hi32(y), (uint32_t)y, sy);
-    fx::Raw rz = fx::split(sf::hi32(z), (uint32_t)z, sz);
-    bool ok = true;
-    if (__any_sync(0xffffffffu, max(max(sx, sy), sz) > 8u)) {
-        rx = fx::splitAny(sf::hi32(x), (uint32_t)x, sx, ok);
-        ry = fx::splitAny(sf::hi32(y), (uint32_t)y, sy, ok);
-        rz = fx::splitAny(sf::hi32(z), (uint32_t)z, sz, ok);
-        ok = __all_sync(0xffffffffu, ok);
-    }
-    r.v = fx::unbias(fx::pack(fx::ffrom(rx.h), fx::ffrom(ry.h)), fx::pack(fx::ffrom(rx.m), fx::ffrom(ry.m)),
-                     fx::pack(fx::ffrom(rx.l), fx::ffrom(ry.l)));
-    r.eh = __fmaf_rn(fx::ffrom(rz.h), 2.0f, -0x1p34f);
-    r.em = fx::ffrom(rz.m) - 0x1p23f;
-    r.el = fx::ffrom(rz.l) - 0x1p23f;
-    return ok;
-}
-
-// the limbs' k - 1 and k + 1 neighbours: (left of x, x), (y, right of y)
-__device__ __forceinline__ void sides(f32x2 v, float edge, int lane, f32x2 &left, f32x2 &right) {
-    const float up = __shfl_up_sync(0xffffffffu, fx::hi(v), 1), dn = __shfl_down_sync(0xffffffffu, fx::lo(v), 1);
-    left = fx::pack(lane == 0 ? edge : up, fx::lo(v));
-    right = fx::pack(fx::hi(v), lane == 31 ? edge : dn);
-}
-
-// volatile: the next row's loads stay where they are, a step ahead of their use
-__device__ __forceinline__ double2 ldGlobal2(const double *p) {
-    double2 v;
-    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ldGlobal(const double *p) {
-    double v;
-    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ void stGlobal(double *p, double v) { asm volatile("st.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory"); }
-__device__ __forceinline__ void stGlobal(double *p, double2 v) {
-    asm volatile("st.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
-}
-__device__ __forceinline__ void stGlobal(int *p, int v) { asm volatile("st.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 
 // strip `local` of loop d: chunk local / nrb, rows (local % nrb) * sr ...; sums: RB * RS doubles of the warp's own
 __device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local, double *sums) {
@@ -150,43 +95,46 @@ __device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local,
     double *const sumItems = d.sumItems, *const minItems = d.minItems;
     int *const locItems = d.locItems;
     int E = fx::E_DEFAULT;
-    auto load = [&](const double *q, HeatRow &r) {
-        r.d = ldGlobal2(q + jo);
-        r.e = ldGlobal(q + eo);
+    auto load = [&](const double *q, rows::Row &r) {
+        r.d = rows::ldGlobal2(q + jo);
+        r.e = rows::ldGlobal(q + eo);
     };
-    HeatRow ra, rc, rd;
+    auto split = [&](rows::Row &r) {
+        if (!needY) r.d.y = r.d.x;  // (not at the load: it would be waited for there)
+        rows::split(r, E);
+    };
+    rows::Row ra, rc, rd;
     load(p, ra);
     load(p + s0, rc);
     load(p + 2 * s0, rd);
-    bool okA = splitRow(ra, E, needY), okC = splitRow(rc, E, needY), okD = splitRow(rd, E, needY);
+    split(ra);
+    split(rc);
+    split(rd);
     int rr = 0;  // rows in the batch
 
     // row i from up, mid, dn; up then takes row i + 2's place
-    auto step = [&](HeatRow &up, HeatRow &mid, HeatRow &dn, bool &okU, bool &okM, bool &okD) -> bool {
-        HeatRow nx;
+    auto step = [&](rows::Row &up, rows::Row &mid, rows::Row &dn) -> bool {
+        rows::Row nx;
         const bool more = left > 1;
         if (more) load(p + 3 * s0, nx);
-        if (__builtin_expect(!(okU && okM && okD), 0)) {  // move the range to end with the three rows' largest value
-            load(p, up);
-            load(p + s0, mid);
-            load(p + 2 * s0, dn);
-            const auto top = [](const HeatRow &h) {
-                return max(max(sf::hi32(sf::bits(h.d.x)), sf::hi32(sf::bits(h.d.y))), sf::hi32(sf::bits(h.e)));
-            };
-            const int e = (int)(__reduce_max_sync(0xffffffffu, max(max(top(up), top(mid)), top(dn))) >> 20) - 8;
-            if (e != E && e >= fx::E_MIN && e <= fx::E_MAX) {
+        if (__builtin_expect(!(up.ok && mid.ok && dn.ok), 0)) {
+            const int e = rows::rangeOf(up, mid, dn, E);
+            if (e != E) {  // move the range
                 E = e;
-                okU = splitRow(up, E, needY);
-                okM = splitRow(mid, E, needY);
-                okD = splitRow(dn, E, needY);
+                load(p, up);
+                load(p + s0, mid);
+                load(p + 2 * s0, dn);
+                split(up);
+                split(mid);
+                split(dn);
             }
         }
         double v0, v1;
-        if (__builtin_expect(okU && okM && okD, 1)) {
+        if (__builtin_expect(up.ok && mid.ok && dn.ok, 1)) {
             fx::Limbs<f32x2> lt, rt;
-            sides(mid.v.h, mid.eh, lane, lt.h, rt.h);
-            sides(mid.v.m, mid.em, lane, lt.m, rt.m);
-            sides(mid.v.l, mid.el, lane, lt.l, rt.l);
+            rows::sides(mid.v.h, mid.eh, lane, lt.h, rt.h);
+            rows::sides(mid.v.m, mid.em, lane, lt.m, rt.m);
+            rows::sides(mid.v.l, mid.el, lane, lt.l, rt.l);
             // ((src[i-1] + src[i+1]) + src[j-1]) + src[j+1]
             const fx::Limbs<f32x2> s = fx::add(fx::add(fx::add(up.v, dn.v), lt), rt);
             // S - 4 src as an integer of the limbs' unit, rounded once
@@ -206,9 +154,9 @@ __device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local,
             if (in1) v1 = q[s0 + 1] + c * ((((q[1] + q[2 * s0 + 1]) + q[s0]) + q[s0 + 2]) - 4.0 * q[s0 + 1]);
         }
         double *out = const_cast<double *>(p) + toOut;
-        if (in0 && in1) stGlobal(out, make_double2(v0, v1));
-        else if (in0) stGlobal(out, v0);
-        else if (in1) stGlobal(out + 1, v1);
+        if (in0 && in1) rows::stGlobal(out, make_double2(v0, v1));
+        else if (in0) rows::stGlobal(out, v0);
+        else if (in1) rows::stGlobal(out + 1, v1);
         // SUM: -0.0 outside the loop
         sums[rr * RS + lane + (lane >> 3)] = (in0 ? v0 : -0.0) + (in1 ? v1 : -0.0);
         // MINLOC: the smallest value's first cell.  Non-negative values below infinity are ordered as their bits are;
@@ -231,9 +179,9 @@ __device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local,
                 who = __ballot_sync(0xffffffffu, h == mh && l == ml);
             }
             if (lane == __ffs(who) - 1) {
-                stGlobal(minItems + item, none ? __builtin_huge_val() : second ? v1 : v0);
-                stGlobal(locItems + 2 * (long)item, row);
-                stGlobal(locItems + 2 * (long)item + 1, (int)j + (second ? 1 : 0));
+                rows::stGlobal(minItems + item, none ? __builtin_huge_val() : second ? v1 : v0);
+                rows::stGlobal(locItems + 2 * (long)item, row);
+                rows::stGlobal(locItems + 2 * (long)item + 1, (int)j + (second ? 1 : 0));
             }
         }
         if (++rr == RB || !more) {
@@ -248,13 +196,13 @@ __device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local,
                 for (int i = 0; i < 8; i += 2 * w) x[i] = x[i] + x[i + w];
             double total = x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
             total = total + __shfl_xor_sync(0xffffffffu, total, 2);
-            if ((lane & 3) == 0 && (lane >> 2) < rr) stGlobal(sumItems + item + ((lane >> 2) + 1 - rr) * nck, total);
+            if ((lane & 3) == 0 && (lane >> 2) < rr) rows::stGlobal(sumItems + item + ((lane >> 2) + 1 - rr) * nck, total);
             __syncwarp();
             rr = 0;
         }
         if (!more) return false;
         up = nx;
-        okU = splitRow(up, E, needY);
+        split(up);
         p += s0;
         item += nck;
         row++;
@@ -262,7 +210,7 @@ __device__ __forceinline__ void heatStrip(const dvmhgb_heat_desc &d, long local,
         return true;
     };
     // three rows a trip, so that the limbs stay where they are
-    while (step(ra, rc, rd, okA, okC, okD) && step(rc, rd, ra, okC, okD, okA) && step(rd, ra, rc, okD, okA, okC)) {
+    while (step(ra, rc, rd) && step(rc, rd, ra) && step(rd, ra, rc)) {
     }
 }
 

@@ -33,6 +33,7 @@
 #include "../../../include/dvmh_gb_kernels.h"
 #include "devinfo.cuh"
 #include "fixlimb.cuh"
+#include "rowlimb.cuh"
 #include "softfp64.cuh"
 
 namespace {
@@ -905,7 +906,7 @@ __device__ __forceinline__ bool inBox2(const Box2 &b, long i, long k) {
 
 template <bool FUSED, int NATIVE>
 __global__ void __launch_bounds__(TX *T2Y) kStencil2(double *A, const double *B, double *Out, Box2 b, long p0,
-                                                      long nstrips, int ichunk, double *items) {
+                                                      long nstrips, int ichunk, double *items, int nitems) {
     __shared__ double sm[T2Y][SW];
     __shared__ double shr[T2Y];
     const int lane = threadIdx.x, ty = threadIdx.y;
@@ -1009,6 +1010,8 @@ __global__ void __launch_bounds__(TX *T2Y) kStencil2(double *A, const double *B,
             for (int w = 1; w < T2Y; w++) r = maxOf(shr[w], r);
             items[blockIdx.x + (long)gridDim.x * blockIdx.y] = r;
         }
+        if (blockIdx.x == 0 && blockIdx.y == 0)  // the items that this launch has no CTA for
+            for (int q = gridDim.x * gridDim.y + ty * TX + lane; q < nitems; q += TX * T2Y) items[q] = -__builtin_huge_val();
     }
 }
 
@@ -1039,6 +1042,8 @@ St2Geom st2Geom(const long lo[2], const long hi[2]) {
     g.grid = dim3((unsigned)gx, (unsigned)gy, 1);
     return g;
 }
+
+#include "stencil2_limb.cuh"
 
 // ---------------------------------------------------------------- copy outside a box
 
@@ -1167,14 +1172,24 @@ void launch3(int variant, const St3Geom &g, double *A, const double *B, double *
 }
 
 template <bool FUSED>
+void launch2L(const St2LGeom &q, double *A, const double *B, double *Out, const Box2 &b, double *items, int nitems,
+              bool rowsToo, cudaStream_t s) {
+    static std::atomic<int> occ[gbdev::MAX_DEVICES];
+    const size_t smem = sizeof(rows::Ring) * 8 * (FUSED ? 2 : 1);
+    gbdev::residentCtas(occ, kStencil2L<FUSED>, 256, smem);  // raises the shared-memory limit
+    kStencil2L<FUSED><<<(unsigned)q.blocks, 256, smem, s>>>(A, B, Out, b, q.c0, q.nchunks, q.sr, q.strips, items, nitems,
+                                                            rowsToo ? 1 : 0);
+}
+
+template <bool FUSED>
 void launch2(int native, const St2Geom &g, double *A, const double *B, double *Out, const Box2 &b, double *items,
-             cudaStream_t s) {
+             int nitems, cudaStream_t s) {
     const int n = FUSED ? 4 : 3;
     native = native < 0 ? 0 : (native > n ? n : native);
     dim3 blk(TX, T2Y);
     switch (native) {
 #define C2(N)                                                                                          \
-    case N: kStencil2<FUSED, (FUSED ? N : (N > 3 ? 3 : N))><<<g.grid, blk, 0, s>>>(A, B, Out, b, g.p0, g.nstrips, g.ichunk, items); break;
+    case N: kStencil2<FUSED, (FUSED ? N : (N > 3 ? 3 : N))><<<g.grid, blk, 0, s>>>(A, B, Out, b, g.p0, g.nstrips, g.ichunk, items, nitems); break;
         C2(0) C2(1) C2(2) C2(3) C2(4)
 #undef C2
     }
@@ -1417,14 +1432,21 @@ int dvmhgb_jac2d_stencil(const double *A, double *B, const long st[2], const lon
     St2Geom g = st2Geom(lo, hi);
     if (!g.ok || !A || !B || !rows16(st, 2) || !aligned16(A) || !aligned16(B)) return -1;
     Box2 b{st[0], ext[0], ext[1], lo[0], lo[1], hi[0], hi[1]};
-    launch2<false>(native, g, (double *)A, nullptr, B, b, nullptr, (cudaStream_t)stream);
+    const St2LGeom q = st2LGeom(lo, hi);
+    if (native >= DVMHGB_JAC2D_STENCIL_LIMBS && q.ok)
+        launch2L<false>(q, const_cast<double *>(A), nullptr, B, b, nullptr, 0, false, (cudaStream_t)stream);
+    else
+        launch2<false>(native, g, (double *)A, nullptr, B, b, nullptr, 0, (cudaStream_t)stream);
     dvmhgb_count_launches(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+// one item per CTA of whichever kernel has more; a launch with fewer CTAs writes the identity to the rest
 long dvmhgb_jac2d_fused_items(const long lo[2], const long hi[2]) {
-    St2Geom g = st2Geom(lo, hi);
-    return (long)g.grid.x * g.grid.y;
+    const St2Geom g = st2Geom(lo, hi);
+    const St2LGeom q = st2LGeom(lo, hi);
+    const long a = (long)g.grid.x * g.grid.y;
+    return q.ok && q.blocks > a ? q.blocks : a;
 }
 
 int dvmhgb_jac2d_fused(double *A, const double *B, double *Bnew, const long st[2], const long ext[2],
@@ -1433,10 +1455,23 @@ int dvmhgb_jac2d_fused(double *A, const double *B, double *Bnew, const long st[2
     if (!g.ok || !A || !B || !Bnew || !items || !rows16(st, 2) || !aligned16(A) || !aligned16(B) || !aligned16(Bnew))
         return -1;
     Box2 b{st[0], ext[0], ext[1], lo[0], lo[1], hi[0], hi[1]};
-    launch2<true>(native, g, A, B, Bnew, b, items, (cudaStream_t)stream);
+    const St2LGeom q = st2LGeom(lo, hi);
+    const int nitems = (int)dvmhgb_jac2d_fused_items(lo, hi);
+    if (native < DVMHGB_JAC2D_FUSED_LIMBS || !q.ok) {
+        launch2<true>(native, g, A, B, Bnew, b, items, nitems, (cudaStream_t)stream);
+        dvmhgb_count_launches(1);
+        if (cudaGetLastError() != cudaSuccess) return -1;
+        return dvmhgb_copy_outside_box(2, B, Bnew, st, ext, lo, hi, stream);
+    }
+    // the kernel copies B's cells beside the box in its chunks' columns; the rows above and below too where they are few
+    // and the chunks cover them
+    const long k0 = q.c0 * 64L, k1 = k0 + q.nchunks * 64L - 1;
+    const long clo[2] = {lo[0], k0}, chi[2] = {hi[0], k1 < ext[1] ? k1 : ext[1] - 1};
+    const bool rowsToo = k0 == 0 && k1 >= ext[1] - 1 && lo[0] <= 4 && ext[0] - 1 - hi[0] <= 4;
+    launch2L<true>(q, A, B, Bnew, b, items, nitems, rowsToo, (cudaStream_t)stream);
     dvmhgb_count_launches(1);
     if (cudaGetLastError() != cudaSuccess) return -1;
-    return dvmhgb_copy_outside_box(2, B, Bnew, st, ext, lo, hi, stream);
+    return rowsToo ? 0 : dvmhgb_copy_outside_box(2, B, Bnew, st, ext, clo, chi, stream);
 }
 
 }  // extern "C"

@@ -17,10 +17,13 @@
 #include "dvmh_gb_kernels.h"
 
 #define R 2
-// FP64 additions per cell of the stencil loop; default count on the FP64 unit
-#define NOPS_STN 3
-#define DEF_STN 3
-#define DEF_FUSED 4
+// variants: additions of a cell on the FP64 unit (0..3 of the stencil loop, 0..4 of the pair), then the FP32 limbs, the
+// fastest from 64^2 to 8192^2 (us, all on the FP64 unit / limbs: the stencil loop 14.7 / 7.2 at 1024^2 and 166 / 67 at
+// 4097^2, the pair 26.9 / 14.1 and 280 / 198, at 130^2 5.4 / 2.7 and 12.0 / 5.0)
+#define N_STN (DVMHGB_JAC2D_STENCIL_LIMBS + 1)
+#define N_FUSED (DVMHGB_JAC2D_FUSED_LIMBS + 1)
+#define DEF_STN DVMHGB_JAC2D_STENCIL_LIMBS
+#define DEF_FUSED DVMHGB_JAC2D_FUSED_LIMBS
 
 namespace {
 
@@ -28,11 +31,11 @@ namespace {
 // the handler (1 update, 2 stencil, 3 the fused pair), its variant number
 constexpr int NDESC = 3;
 const float *variantDesc(int handler) {
-    static float d[3][(NOPS_STN + 2) * NDESC];
+    static float d[3][N_FUSED * NDESC];
     static bool ready = false;
     if (!ready) {
         for (int h = 1; h <= 3; h++)
-            for (int v = 0; v < NOPS_STN + 2; v++) {
+            for (int v = 0; v < N_FUSED; v++) {
                 d[h - 1][v * NDESC] = 2, d[h - 1][v * NDESC + 1] = (float)h, d[h - 1][v * NDESC + 2] = (float)v;
             }
         ready = true;
@@ -104,7 +107,7 @@ extern "C" void loop_jac2d_stn_cuda(DvmType *pLoopRef, DvmType A_hdr[], DvmType 
     dim3 threads(0, 0, 0);
     cudaStream_t stream;
     dvmh_loop_cuda_get_config_C(loop_ref, 0, 0, &threads, &stream, 0);
-    check(dvmhgb_jac2d_stencil(A.base, B.base, A.st, A.ext, lo, hi, dvmhgb_loop_variant_desc(loop_ref, NOPS_STN + 1, DEF_STN, variantDesc(2), NDESC), stream), "loop_jac2d_stn_cuda");
+    check(dvmhgb_jac2d_stencil(A.base, B.base, A.st, A.ext, lo, hi, dvmhgb_loop_variant_desc(loop_ref, N_STN, DEF_STN, variantDesc(2), NDESC), stream), "loop_jac2d_stn_cuda");
 }
 
 // refs[0]: the update loop (A_hdr, B_hdr, eps_ptr), refs[1]: the stencil loop (A2_hdr, B2_hdr)
@@ -133,7 +136,7 @@ extern "C" void loop_jac2d_fused_cuda(DvmType refs[2], DvmType A_hdr[], DvmType 
     dvmh_loop_cuda_red_prepare_C(upd, 1, dvmhgb_jac2d_fused_items(lo, hi), 0);
     double *Bnew = (double *)dvmhgb_loop_alt_buffer(stn, B_hdr);
     check(dvmhgb_jac2d_fused(A.base, B.base, Bnew, A.st, A.ext, lo, hi, eps_grid,
-                             dvmhgb_loop_variant_desc(upd, NOPS_STN + 2, DEF_FUSED, variantDesc(3), NDESC), stream),
+                             dvmhgb_loop_variant_desc(upd, N_FUSED, DEF_FUSED, variantDesc(3), NDESC), stream),
           "loop_jac2d_fused_cuda");
     dvmh_loop_cuda_red_finish_C(upd, 1);
 }

@@ -97,6 +97,11 @@ int dvmhgb_jac3d_fused(double *A, const double *B, double *Bnew, const long st[3
                        const long lo[3], const long hi[3], double *items, int native, void *stream);
 
 /* ---- Jacobi 2-D (examples/Jacobi/jac2d.c:49-64, FP64) ---- */
+/* native as above for the additions of a cell on the FP64 unit (stencil 0..3,
+ * fused 0..4, the rest on the integer pipe); DVMHGB_JAC2D_*_LIMBS and above: the
+ * sums on FP32 limbs, |B - A| on the FP64 unit */
+#define DVMHGB_JAC2D_STENCIL_LIMBS 4
+#define DVMHGB_JAC2D_FUSED_LIMBS 5
 long dvmhgb_jac2d_update_items(const long lo[2], const long hi[2]);
 int dvmhgb_jac2d_update(double *A, const double *B, const long st[2], const long lo[2], const long hi[2],
                         double *items, int native, void *stream);
