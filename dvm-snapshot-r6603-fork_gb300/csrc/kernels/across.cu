@@ -41,6 +41,7 @@
 #include "../../../include/dvmh_gb.h"
 #include "../../../include/dvmh_gb_kernels.h"
 #include "devinfo.cuh"
+#include "fixlimb.cuh"
 
 namespace {
 
@@ -568,6 +569,9 @@ int sweepStream(double *A, const Geo &g0, const double *wDev, double *items, voi
 
 // ---------------------------------------------------------------- hyperplane tiles (variants 4 and 5)
 //
+// Variant 4 hands out tiles of 4 x 8 rows, one per warp; variant 5 walks columns
+// of tiles of 16 x 8 rows, one per CTA (below, "columns").
+//
 // The tiles above are boxes: inside one, lane (li, lj) starts li + lj steps
 // late, so a 4 x 8 x TK tile takes TK + 10 steps for TK positions per lane, and
 // on GB300 an FP64 warp instruction costs the same whatever its active lanes.
@@ -708,6 +712,21 @@ __device__ __forceinline__ bool hypWait(const int *f, int want, int *status, uns
         __nanosleep(64);
     }
     return true;
+}
+
+// the same by one thread of a CTA; the value seen, -1 once the limit ran out
+__device__ __forceinline__ int hypWaitFor(const int *f, int want, int *status, unsigned *counter, long limit) {
+    long n = 0;
+    int v;
+    while ((v = ldAcquire(f)) < want) {
+        if (++n > limit) {
+            atomicExch(status, ERR_SOR_TIMEOUT);
+            atomicOr(counter, 0x80000000u);  // no warp takes another column
+            return -1;
+        }
+        __nanosleep(64);
+    }
+    return v;
 }
 
 __device__ __forceinline__ double ldH(const double *A, const HGeo &g, long i, long j, long k) {
@@ -903,169 +922,346 @@ __global__ void __launch_bounds__(NT) kSorHyp(double *A, HGeo g, const double *w
     }
 }
 
-// CTA tiles: TIc x TJc rows, one thread per row (TIc * TJc / 32 warps), one tile per CTA.  Fewer, larger
-// tiles shorten the chain of tile planes (a + b + c) a sweep has to go through; the tile's warps take their
-// steps in lockstep (a CTA barrier per step), each on its own SM sub-partition.
-template <int G, int TIc, int TJc>
-struct HypC {
-    static constexpr int NTc = TIc * TJc;
-    static constexpr int SIc = TIc + 2, SJc = TJc + 2;
-    static constexpr int SKP = G + 3;  // window: positions 0 .. G + 1 (odd stride: banks)
-    static constexpr int BOX = SIc * SJc * SKP;
-    static constexpr int SQS = 2 * G + 1;
+// ---- columns of hyperplane tiles (variant 5, the default)
+//
+// A CTA of WI = 4 warps walks a column (a, b) of 16 x 8 rows from its first tile to its last, its warps in lockstep (a
+// barrier per step).  What one tile leaves to the next stays in the CTA: the rows' last new values, the squares of an
+// open part, the window.  So the only dependences between CTAs are (a-1, b) and (a, b-1), tile c of each before tile c
+// here, told by one progress word per column; columns are handed out along the diagonals a + b (topological, and no
+// more CTAs than the GPU holds at once).  The next hyperplanes are copied (cp.async) during a tile's steps.
+//
+// A step's sum of six neighbours runs on FP32 limbs (fixlimb.cuh): the FP64 unit takes an instruction per 62 - 76
+// cycles from a warp, a limb addition 29, and the unit is left to the two products, the update and the residual, 6
+// instructions a step instead of 11.  A step with a value outside the limbs' range (nine binades around the largest
+// of the tile before) sums on the FP64 unit; after a tile with three such steps, or with negative values, the next eight
+// tiles do.
+//
+// What bounds it: the chain of tile planes a + b + c (52 for 97^3, 214 for 384^3) at about 11,000 cycles each: 8 steps
+// of 870 - 950 (the dependent chain of split, five additions, assembly, two FP64 operations and the barrier), 700 for
+// the faces, 1,100 to store and publish, 1,000 until the next column sees it.  Measured per sweep (values in one
+// range), against tiles of one warp (variant 4) and one tile of 16 x 8 rows per CTA and hand-out, with all sums on
+// FP64: 97^3 295 us (366, 316), 384^3 1770 us (2035, 2037).  With signed values: 97^3 322 us (365), 384^3 2250 us (2035):
+// variant 4 remains for large boxes of those.  What did not help: limbs kept in shared memory and split once by their
+// producer (unrolled or not, 288 and 1788 us), four CTAs per SM (1946 us at 384^3), 32 x 8 rows (2166 us), 8 x 8 (1749
+// us; 320 us at 97^3), unrolled steps (instruction cache: 1821 - 1880 us).
+
+template <int G, int WI>
+struct HypCol {
+    static_assert(TJ == G && TI * TJ == 32, "the staging lanes take 8 positions of 4 rows");
+    static constexpr int RING = 3 * G;                                    // hyperplanes of a row: c - 1, c, c + 1
+    static constexpr int SKP = RING + 1;                                  // odd ...
+    static constexpr int RS = (SJ * SKP + 7) / 16 * 16 + 8;               // ... and 8 mod 16: no bank conflicts
+    static constexpr int NTc = 32 * WI;
+    static constexpr int BOX = (TI * WI + 2) * RS;
+    static constexpr int SQS = 2 * G + G;                                 // a lane's squares of two parts, tree nodes
     static constexpr size_t SMEM = sizeof(double) * (BOX + NTc * SQS);
+    static_assert(RS >= SJ * SKP, "rows overlap");
 };
 
-template <int G, int TIc, int TJc>
-__global__ void __launch_bounds__(TIc * TJc, 4) kSorHypCta(double *A, HGeo g, const double *wPtr, int *flags,
-                                                        unsigned *counter, const unsigned long long *table,
-                                                        double *carry, double *items, int *status, Bound bound) {
-    using H = HypC<G, TIc, TJc>;
-    constexpr int SKP = H::SKP, SJc = H::SJc, RS = SJc * SKP, NTc = H::NTc;
-    extern __shared__ double sm[];  // box [SIc][SJc][SKP], then leaves [NTc][SQS]
-    __shared__ long tileIdx;
-    const int tid = threadIdx.x, li = tid / TJc, lj = tid % TJc;
-    double *box = sm;
-    double *sq = sm + H::BOX + tid * H::SQS;
+// a tile with MISSES steps that met values outside the limbs' range has the next NATIVE tiles done by the FP64 unit
+constexpr int MISSES = 3, NATIVE = 8;
+
+// x on FP32 limbs; clears ok where it is neither +0 nor in the range of E
+__device__ __forceinline__ fx::Limbs<float> limbs(double x, int E, bool &ok) {
+    const uint64_t X = sf::bits(x);
+    const fx::Raw r = fx::splitAny(sf::hi32(X), (uint32_t)X, fx::place(sf::hi32(X), E), ok);
+    return fx::unbias(fx::ffrom(r.h), fx::ffrom(r.m), fx::ffrom(r.l));
+}
+
+// the range of nine binades, with one binade above the largest value seen (high word `big`) for those of the next tile
+__device__ __forceinline__ int rangeAround(unsigned big) {
+    const int top = (int)(big >> 20);
+    return top < fx::E_MIN + 7 ? fx::E_MIN : top > fx::E_MAX + 7 ? fx::E_MAX : top - 7;
+}
+
+__device__ __forceinline__ unsigned highWord(double x) { return sf::hi32(sf::bits(x)); }
+
+// asynchronous copy of one double, 0.0 where !ok (any: some address inside the array)
+__device__ __forceinline__ void copyCell(double *dst, const double *src, bool ok, const double *any) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(ok ? src : any), "r"(ok ? 8 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copiesDone() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// number of columns (a, b) with a + b < s
+__device__ __forceinline__ long columnsBefore(long s, long na, long nb) {
+    const auto tri = [](long x) { return x > 0 ? x * (x + 1) / 2 : 0; };
+    return tri(s) - tri(s - na) - tri(s - nb) + tri(s - na - nb);
+}
+
+// d * d inside the loop, -0.0 outside
+__device__ __forceinline__ double leaf(double d, bool in) { return (in ? d : -0.0) * (in ? d : 0.0); }
+
+template <int G, int WI>
+__global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g, const double *wPtr, int *prog,
+                                                               unsigned *counter, double *items, int *status,
+                                                               Bound bound) {
+    using H = HypCol<G, WI>;
+    constexpr int SKP = H::SKP, RS = H::RS, RING = H::RING, NTc = H::NTc;
+    extern __shared__ double sm[];  // box [TI WI + 2][RS], then squares and nodes [SQS][NTc]
+    __shared__ long sIdx;
+    __shared__ bool sAhead[2];
+    const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5, li = lane / TJ, lj = lane % TJ;
+    const int lr = li, lp = lj;     // staging: a lane copies position lp of rows lr, lr + 4, ...
+    double *box = sm + wi * TI * RS;                   // the warp's rows and their faces
+    double *sq = sm + H::BOX + tid;
+    double *x = box + (li + 1) * RS + (lj + 1) * SKP;  // the lane's row; hyperplane h at position h mod RING
     const double w = *wPtr;
     const double c1 = 1.0 - w, c2 = w / 6.0;  // loop invariants, rounded as in the source expression
     const int nk = (int)g.nk;
+    // rk (k - lo2) of the cells stored in the array: [rlo, rhi), clamped well outside every window
+    const int rlo = (int)-(g.lo2 < (1L << 30) ? g.lo2 : 1L << 30);
+    const int rhi = (int)(g.e2 - g.lo2 < (1L << 30) ? g.e2 - g.lo2 : 1L << 30);
+    const int kofs = (int)(g.lo2 & 63);       // k's position in its 64-wide chunk at rk = 0
     while (true) {
-        if (tid == 0) tileIdx = (long)atomicAdd(counter, 1u) + bound.firstIndex;  // >= 2^31 once a CTA has failed
-        __syncthreads();  // the index; and the previous tile's last box reads are done
-        const long idx = tileIdx;
-        if (idx >= g.ntiles) break;
-        const unsigned long long tv = table[idx];
-        const long a = (long)(tv >> 42), b = (long)((tv >> 21) & 0x1fffff), c = (long)(tv & 0x1fffff);
-        const long ra = TIc * a, rb = TJc * b, hc = G * c;
-        // 1. before the wait: rows qi 1..TIc+1, qj 1..TJc+1, positions 1 .. G+1 (old values)
-        {
-            constexpr int NV = (H::SIc - 1) * (SJc - 1) * (G + 1), NL = (NV + NTc - 1) / NTc;
-            double v[NL];
-#pragma unroll
-            for (int u = 0; u < NL; u++) {
-                const int q = u * NTc + tid, r = q / (G + 1), p = 1 + q % (G + 1);
-                const int qi = 1 + r / (SJc - 1), qj = 1 + r % (SJc - 1);
-                const long fi = ra - 1 + qi, fj = rb - 1 + qj;
-                v[u] = q < NV ? ldH(A, g, g.lo0 + fi, g.lo1 + fj, g.lo2 + hc - fi - fj - 1 + p) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < NL; u++) {
-                const int q = u * NTc + tid, r = q / (G + 1), p = 1 + q % (G + 1);
-                const int qi = 1 + r / (SJc - 1), qj = 1 + r % (SJc - 1);
-                if (q < NV) box[(qi * SJc + qj) * SKP + p] = v[u];
-            }
+        if (tid == 0) sIdx = (long)atomicAdd(counter, 1u) + bound.firstIndex;  // >= 2^31 once a warp has failed
+        __syncthreads();
+        const long idx = sIdx;
+        if (idx >= g.na * g.nb) break;
+        long sd = 0;  // the last diagonal with columnsBefore(sd) <= idx
+        for (long top = g.na + g.nb - 2; sd < top;) {
+            const long mid = (sd + top + 1) / 2;
+            if (columnsBefore(mid, g.na, g.nb) <= idx) sd = mid;
+            else top = mid - 1;
         }
-        // 2. wait for the five predecessors (bounded); the barrier orders the acquiring threads' loads
-        //    before every thread's face loads
-        int fail = 0;
-        if (tid < 5) {
-            // threads 0..4: (a-1,b,c), (a-1,b,c-1), (a,b-1,c), (a,b-1,c-1), (a,b,c-1)
-            const long pa = a - (tid < 2), pb = b - (tid == 2 || tid == 3), pc = c - (tid == 1 || tid == 3 || tid == 4);
-            if (pa >= 0 && pb >= 0 && pc >= hypCmin<G>(g, pa, pb) && pc <= hypCmax<G>(g, pa, pb) &&
-                !hypWait(flags + (pa * g.nb + pb) * g.ncg + pc, 1, status, counter, bound.pollLimit))
-                fail = 1;
-        }
-        if (__syncthreads_or(fail)) return;
+        const long a = (sd - (g.nb - 1) > 0 ? sd - (g.nb - 1) : 0) + idx - columnsBefore(sd, g.na, g.nb), b = sd - a;
+        const long ra = TI * (WI * a + wi), rb = TJ * b;  // the warp's first row
+        const int cmin = (int)hypCmin<G>(g, a, b), cmax = (int)hypCmax<G>(g, a, b);
+        // thread 0 waits for column (a-1, b), thread 1 for (a, b-1)
+        const bool waits = tid == 0 ? a > 0 : tid == 1 && b > 0;
+        const long pa = a - (tid == 0), pb = b - (tid == 1);
+        const int *before = prog + pa * g.nb + pb;
+        const int plast = waits ? (int)hypCmax<G>(g, pa, pb) : 0;
+        int seen = 0;
+        // the warp's rows and its +i / +j faces, 4 rows x 8 positions a copy: 8 copies of own rows, 2 of the +i
+        // face, 1 of the +j face.  rk of copy u at hyperplane h: h + q0 - its row's distance
+        const int q0 = lp - (int)(ra + rb) - lr;
+        double *src = A + (g.lo0 + ra) * g.s0 + (g.lo1 + rb + lr) * g.s1 + g.lo2 + q0;
+        const double *srcJ = A + (g.lo0 + ra + lr) * g.s0 + (g.lo1 + rb + TJ) * g.s1 + g.lo2 + q0 - TJ;
+        const bool okJ0 = g.lo1 + rb + lr < g.e1, okJ4 = g.lo1 + rb + 4 + lr < g.e1;
+        const bool okJ = g.lo1 + rb + TJ < g.e1 && g.lo0 + ra + lr < g.e0;
+        const bool inJ0 = g.lo1 + rb + lr <= g.hi1, inJ4 = g.lo1 + rb + 4 + lr <= g.hi1;
+        const int rowsS = (int)(g.hi0 - g.lo0 - ra + 1 < TI ? g.hi0 - g.lo0 - ra + 1 : TI);
+        const int rowsI = (int)(g.e0 - g.lo0 - ra < 5 ? g.e0 - g.lo0 - ra : 5);
+        double *dst = box + RS + (1 + lr) * SKP + lp, *dstJ = box + (1 + lr) * RS + (TJ + 1) * SKP + lp;
+        auto stage = [&](int c) {
+            const int at = c % 3 * G, h = c * G;
+#pragma unroll
+            for (int u = 0; u < 10; u++) {
+                if (u >= 8 && wi != WI - 1) break;  // the +i face: the next warp's rows
+                const int qi = u / 2, qj = u % 2 * 4, rk = h + q0 - qi - qj;
+                copyCell(dst + at + qi * RS + qj * SKP, src + h + qi * (g.s0 - 1) + qj * (g.s1 - 1),
+                         (qj ? okJ4 : okJ0) && qi < rowsI && rk >= rlo && rk < rhi, A);
+            }
+            const int rk = h + q0 - TJ;
+            copyCell(dstJ + at, srcJ + h, okJ && rk >= rlo && rk < rhi, A);
+        };
+        // the -i face (rows 0, 1..8: two loads) and the -j face (rows 1..4, 0: one load) at tile c's hyperplanes
+        double f0, f1, f2;
+        const bool okI = g.lo0 + ra >= 1, okK = g.lo1 + rb >= 1 && g.lo0 + ra + lr < g.e0;
+        const double *srcI = src - (g.s0 - 1), *srcK = srcJ - (TJ + 1) * (g.s1 - 1);
+        auto faces = [&](int c) {
+            const int h = c * G, r0 = h + q0 + 1, r1 = r0 - 4, r2 = h + q0 + 1;
+            f0 = wi == 0 && okI && okJ0 && r0 >= rlo && r0 < rhi ? __ldcg(srcI + h) : 0.0;
+            f1 = wi == 0 && okI && okJ4 && r1 >= rlo && r1 < rhi ? __ldcg(srcI + h + 4 * (g.s1 - 1)) : 0.0;
+            f2 = okK && r2 >= rlo && r2 < rhi ? __ldcg(srcK + h) : 0.0;
+        };
         const long ri = ra + li, rj = rb + lj, i = g.lo0 + ri, j = g.lo1 + rj;
         const bool row = i <= g.hi0 && j <= g.hi1;
-        const int rk0 = (int)(hc - ri - rj);
-        const long k0 = g.lo2 + rk0;
-        const long m = hypFloor<G>(k0);                       // the part boundary at or below k0
-        const int dl = (int)(k0 - m);
-        const long rowIdx = row ? (i - g.lo0) * g.nj + (j - g.lo1) : 0;
-        const bool first = c == hypCmin<G>(g, a, b);
-        const bool res = row && k0 <= g.hi2;
-        // 3. the -i face rows (0, 1..TJc), the -j face rows (1..TIc, 0) at positions 0 .. G-1, the own rows at
-        //    0, and the carried differences
-        double cin[G - 1];
-        {
-            constexpr int NV = (TIc + TJc) * G, NL = (NV + NTc - 1) / NTc;
-            double v[NL];
-#pragma unroll
-            for (int u = 0; u < NL; u++) {
-                const int q = u * NTc + tid, r = q / G, p = q % G;
-                const int qi = r < TJc ? 0 : r - TJc + 1, qj = r < TJc ? r + 1 : 0;
-                const long fi = ra - 1 + qi, fj = rb - 1 + qj;
-                v[u] = q < NV ? ldH(A, g, g.lo0 + fi, g.lo1 + fj, g.lo2 + hc - fi - fj - 1 + p) : 0.0;
-            }
-            const double k0v = ldH(A, g, i, j, k0 - 1);
-#pragma unroll
-            for (int q = 0; q < G - 1; q++)
-                cin[q] = res && !first && q < dl ? __ldcg(carry + q * g.rows + rowIdx) : 0.0;
-#pragma unroll
-            for (int u = 0; u < NL; u++) {
-                const int q = u * NTc + tid, r = q / G, p = q % G;
-                const int qi = r < TJc ? 0 : r - TJc + 1, qj = r < TJc ? r + 1 : 0;
-                if (q < NV) box[(qi * SJc + qj) * SKP + p] = v[u];
-            }
-            box[((li + 1) * SJc + lj + 1) * SKP] = k0v;
-        }
+        int rk0 = cmin * G - (int)(ri + rj);  // the row's rk at step 0
+        double *it = items + (row ? ((i - g.lo0) * g.nj + (j - g.lo1)) * g.nparts : 0);
+        if (row)
+            for (int q = 0; q < (rk0 + kofs) >> 3 && q < g.nparts; q++) it[q] = -0.0;  // parts before the column
+        stage(cmin);
+        stage(cmin + 1);
+        double prev = ldH(A, g, i, j, g.lo2 + rk0 - 1);
+        for (int q = 0; q < 2 * G; q++) sq[NTc * q] = -0.0;
+        // values of the first hyperplanes choose the first range
+        copiesDone();
         __syncthreads();
-        double *x = box + ((li + 1) * SJc + (lj + 1)) * SKP + 1;  // x[t]: position t + 1
-        double dv[G];
-        // 4. the dependent chain: G steps, one thread per row, the CTA in lockstep
-#pragma unroll
-        for (int t = 0; t < G; t++) {
-            const int rk = rk0 + t;
-            dv[t] = 0.0;
-            if (row && rk >= 0 && rk < nk) {
-                const double old = x[t];
-                // A[i-1] + A[i+1] + A[j-1] + A[j+1] + A[k-1] + A[k+1], left to right
-                const double s = ((((x[t - RS - 1] + x[t + RS + 1]) + x[t - SKP - 1]) + x[t + SKP + 1]) + x[t - 1]) +
-                                 x[t + 1];
-                const double nv = c1 * old + c2 * s;
-                x[t] = nv;
-                dv[t] = nv - old;
-            }
-            __syncthreads();
-        }
-        // 5. store what the successors read (rows li = TIc-1 and lj = TJc-1, the last position of the others,
-        //    the carried differences), release the successors, then store the other cells
-        auto store = [&](int r, int p) {
-            const int qi = r / TJc, qj = r % TJc;
-            const long ii = ra + qi, jj = rb + qj, rk = hc - ii - jj + p - 1;
-            if (g.lo0 + ii <= g.hi0 && g.lo1 + jj <= g.hi1 && rk >= 0 && rk < nk)
-                A[(g.lo0 + ii) * g.s0 + (g.lo1 + jj) * g.s1 + g.lo2 + rk] = box[((qi + 1) * SJc + qj + 1) * SKP + p];
+        unsigned big = 0;
+        for (int q = 0; q < 2 * G; q++) big = max(big, highWord(x[(cmin * G + q) % RING]));
+        big = __reduce_max_sync(0xffffffffu, big);
+        int E = rangeAround(big), misses = 0, native = big >> 31 ? NATIVE : 0;
+        int at = cmin % 3 * G;  // position of the tile's first hyperplane
+        bool oki = true, okj = true, okk = true;
+        double old = x[at], kp = x[at + 1];
+        unsigned some = 0;  // high words of the old terms
+        x[at ? at - 1 : RING - 1] = prev;
+        fx::Limbs<float> ip, jp, kl;  // the +i, +j and +k terms of the next step
+        auto terms = [&](int q, double kq) {
+            const double iq = x[q + RS], jq = x[q + SKP];
+            oki = okj = okk = true;
+            ip = limbs(iq, E, oki);
+            jp = limbs(jq, E, okj);
+            kl = limbs(kq, E, okk);
+            some = highWord(iq) | highWord(jq) | highWord(kq);
         };
-        {
-            constexpr int N1 = TJc * G, N2 = N1 + (TIc - 1) * G, NE = N2 + (TIc - 1) * (TJc - 1);
+        terms(at + 1, kp);
+        bool ahead = false;     // this tile's -i / -j faces are in f0, f1, f2
+        double dv = 0.0, root = 0.0;  // new value - old value of the last step; the last tree node
+        bool actd = false;            // the last step's cell lies in the loop
+        double sqv = -0.0;            // the square of the step before that
+        for (int c = cmin; c <= cmax; c++, rk0 += G) {
+            // 1. the -i / -j faces: tile c of the two columns before this one (bounded wait)
+            if (!ahead) {
+                int fail = 0;
+                if (waits) {
+                    const int want = (c < plast ? c : plast) + 1;
+                    if (seen < want) {
+                        seen = hypWaitFor(before, want, status, counter, bound.pollLimit);
+                        fail = seen < 0;
+                    }
+                }
+                // also orders the acquiring threads' loads before every thread's face loads
+                fail = __syncthreads_or(fail);
+                if (fail) {
+                    copiesDone();
+                    return;
+                }
+                faces(c);
+                if (c == cmin && lane < TI + TJ && (wi == 0 || lane >= TJ)) {  // and the hyperplane before the column
+                    const int qi = lane < TJ ? 0 : lane - TJ + 1, qj = lane < TJ ? lane + 1 : 0;
+                    const long fi = ra - 1 + qi, fj = rb - 1 + qj;
+                    box[qi * RS + qj * SKP + (at ? at - 1 : RING - 1)] =
+                        ldH(A, g, g.lo0 + fi, g.lo1 + fj, g.lo2 + (long)cmin * G - fi - fj - 1);
+                }
+            }
+            if (wi == 0) {
+                box[(1 + lr) * SKP + at + lp] = f0;
+                box[(5 + lr) * SKP + at + lp] = f1;
+            }
+            box[(1 + lr) * RS + at + lp] = f2;
+            copiesDone();
+            if (tid < 2) sAhead[tid] = !waits || seen > (c + 1 < plast ? c + 1 : plast);
+            __syncthreads();
+            // the next tile's faces already: the columns before this one are further ahead
+            ahead = c < cmax && sAhead[0] && sAhead[1];
+            if (ahead) faces(c + 1);
+            // 2. the dependent chain: G steps, every lane on its own row.  The terms that do not depend on the step
+            //    before (+i, +j, +k of the next step, the part the last tile closed) fill the FP64 unit's latencies
+            big = 0;
+            int pm = at ? at - 1 : RING - 1, p0 = at;
+            const int half = (rk0 + kofs - G) & G;  // where the squares of the part that the last tile closed are
+            const auto step = [&](int t, auto limbs6) {
+                constexpr bool LIMB = decltype(limbs6)::value;
+                const int rk = rk0 + t;
+                const int pp = p0 + 1 == RING ? 0 : p0 + 1, p2 = pp + 1 == RING ? 0 : pp + 1;
+                const bool act = row && (unsigned)rk < (unsigned)nk;
+                // A[i-1] + A[i+1] + A[j-1] + A[j+1] + A[k-1] + A[k+1], left to right
+                const double im = x[pm - RS], jm = x[pm - SKP];
+                // a node of the closed part's pairwise tree and the square of the step before; what the last step
+                // computed of them is stored now, so that nothing waits for the FP64 unit here
+                sq[NTc * (2 * G + (t + G - 1) % G)] = root;
+                sq[NTc * ((rk - 2 + kofs) & (2 * G - 1))] = sqv;
+                const int node = t < 4 ? half + 2 * t : t < 6 ? 2 * G + 2 * t - 8 : 2 * G + 4;
+                root = sq[NTc * node] + sq[NTc * node + NTc];
+                sqv = leaf(dv, actd);
+                const double cold = c1 * old;
+                double s;
+                if (LIMB) {
+                    bool ok = oki && okj && okk;
+                    fx::Limbs<float> sl = fx::add(limbs(im, E, ok), ip);
+                    sl = fx::add(sl, limbs(jm, E, ok));
+                    sl = fx::add(sl, jp);
+                    sl = fx::add(sl, limbs(prev, E, ok));
+                    sl = fx::plus(sl, kl);
+                    // six zeros, or a sum that can be assembled
+                    s = some | highWord(im) | highWord(jm) | highWord(prev) ? fx::sumDouble(sl, E) : 0.0;
+                    if (__any_sync(0xffffffffu, act && !ok)) {
+                        misses++;
+                        s = im;
+                        // a loop: as straight code the compiler issues these FP64 instructions, predicated off, always
+#pragma unroll 1
+                        for (int q = 0; q < 5; q++)
+                            s = s + x[q == 0 ? pp + RS : q == 1 ? pm - SKP : q == 2 ? pp + SKP : q == 3 ? pm : pp];
+                    }
+                } else {
+                    s = ((((im + x[pp + RS]) + jm) + x[pp + SKP]) + prev) + kp;
+                }
+                if (act) big = max(max(max(highWord(im), highWord(jm)), highWord(kp)), big);
+                const double nv = cold + c2 * s;
+                const double kn = x[p2];
+                if (LIMB) terms(p2, kn);
+                if (act) x[p0] = nv;
+                __syncthreads();
+                dv = nv - old;
+                actd = act;
+                prev = act ? nv : old;
+                old = kp;
+                kp = kn;
+                pm = p0;
+                p0 = pp;
+                if (t == 0 && c < cmax) stage(c + 2);  // over the hyperplanes of c - 1, read for the last time
+            };
+            if (native > 0) {
+#pragma unroll 1
+                for (int t = 0; t < G; t++) step(t, std::false_type());
+            } else {
+#pragma unroll 1
+                for (int t = 0; t < G; t++) step(t, std::true_type());
+            }
+            // 3. store what the successors read -- the rows li = 3 and lj = 7 -- and publish the tile, then store its
+            //    other cells (read by no other column of this sweep)
+            auto store = [&](int qi, int qj) {  // 4 rows x 8 positions
+                if ((qj ? inJ4 : inJ0) && qi < rowsS && (unsigned)(c * G + q0 - qi - qj) < (unsigned)nk)
+                    *(src + c * G + qi * (g.s0 - 1) + qj * (g.s1 - 1)) =
+                        box[(1 + qi) * RS + (1 + qj + lr) * SKP + at + lp];
+            };
+            const bool edge = wi == WI - 1;  // the warp with the tile's last row
+            if (edge) {
+                store(TI - 1, 0);
+                store(TI - 1, 4);
+            }
+            if (lr == 3) {
 #pragma unroll
-            for (int u = 0; u < (NE + NTc - 1) / NTc; u++) {
-                const int e = u * NTc + tid;
-                if (e < N1) store((TIc - 1) * TJc + e / G, 1 + e % G);
-                else if (e < N2) store(((e - N1) / G) * TJc + TJc - 1, 1 + (e - N1) % G);
-                else if (e < NE) store(((e - N2) / (TJc - 1)) * TJc + (e - N2) % (TJc - 1), G);
+                for (int qi = 0; qi < TI; qi++)
+                    if (qi < TI - 1 || !edge) store(qi, 4);
+            }
+            // the barrier orders every thread's stores before thread 0's release at GPU scope, which publishes
+            // them (release cumulativity) without a sequentially consistent fence in every thread
+            __syncthreads();
+            if (tid == 0) stRelease(prog + a * g.nb + b, c + 1);
+#pragma unroll
+            for (int qi = 0; qi < TI; qi++)
+                if (qi < TI - 1 || !edge) {
+                    store(qi, 0);
+                    if (lr < 3) store(qi, 4);
+                }
+            // 4. the part closed a tile ago
+            const int part = (rk0 + kofs - G) >> 3;
+            if (row && c > cmin && part >= 0 && part < g.nparts) it[part] = root;
+            // 5. the range for the next tile
+            big = __reduce_max_sync(0xffffffffu, big);
+            at = at + G == RING ? 0 : at + G;
+            // values outside the limbs' range: the next tiles on the FP64 unit
+            if (native > 0) native--;
+            if (misses >= MISSES || big >> 31) native = NATIVE;
+            misses = 0;
+            if (native == 0) {
+                if (big) E = rangeAround(big);
+                terms(at + 1, kp);
             }
         }
+        // the column's last two parts, then -0.0 to the end
+        sq[NTc * ((rk0 - 2 + kofs) & (2 * G - 1))] = sqv;
+        sq[NTc * ((rk0 - 1 + kofs) & (2 * G - 1))] = leaf(dv, actd);
+        if (row) {
+            const int last = (rk0 - G + kofs) >> 3;
+            for (int q = last < 0 ? 0 : last; q < g.nparts; q++) {
+                double v[G];
 #pragma unroll
-        for (int t = 1; t < G; t++)  // position t is leaf t - G + dl of the next part
-            if (res && t - G + dl >= 0) carry[(t - G + dl) * g.rows + rowIdx] = dv[t];
-        // the CTA barrier orders every thread's stores before thread 0's release at GPU scope
-        __syncthreads();
-        if (tid == 0) stRelease(flags + (a * g.nb + b) * g.ncg + c, 1);
+                for (int p = 0; p < G; p++)
+                    v[p] = q < last + 2 && q * G + p - kofs < nk ? sq[NTc * ((q * G + p) & (2 * G - 1))] : -0.0;
 #pragma unroll
-        for (int u = 0; u < G; u++) {  // rows li < TIc-1, lj < TJc-1 at positions 1 .. G-1
-            const int q = u * NTc + tid, r = q / G, p = 1 + q % G;
-            if (r / TJc < TIc - 1 && r % TJc < TJc - 1 && p < G) store(r, p);
-        }
-        // 6. the residual, off the chain (per thread, as in the warp tiles)
-        if (res) {
+                for (int o = 1; o < G; o *= 2)
 #pragma unroll
-            for (int q = 0; q < G - 1; q++)
-                if (q < dl) sq[q] = cin[q];
-#pragma unroll
-            for (int t = 0; t < G; t++) sq[dl + t] = dv[t];
-            const long P = m / G - g.kc0;
-            double *it = items + rowIdx * g.nparts;
-            if (first)
-                for (long q = 0; q < P && q < g.nparts; q++) it[q] = -0.0;
-            if (P >= 0 && P < g.nparts) it[P] = hypTree<G>(sq, m, g.lo2, g.hi2);
-            if (k0 + G - 1 >= g.hi2) {
-                if (P + 1 >= 0 && P + 1 < g.nparts) it[P + 1] = hypTree<G>(sq + G, m + G, g.lo2, g.hi2);
-                for (long q = P + 2 > 0 ? P + 2 : 0; q < g.nparts; q++) it[q] = -0.0;
+                    for (int p = 0; p < G; p += 2 * o) v[p] = v[p] + v[p + o];
+                it[q] = v[0];
             }
         }
+        __syncthreads();  // the box and the index are reused for the next column
     }
 }
 
@@ -1120,8 +1316,8 @@ HypScratch hypScratch(const HGeo &g) {
     return s;
 }
 
-// one hyperplane sweep: the tile list, then the persistent wavefront.  cta: tiles of CTA_TI x CTA_TJ rows, one
-// per CTA (kSorHypCta); else tiles of 4 x 8 rows, one per warp (kSorHyp)
+// one hyperplane sweep.  cta: columns of CTA_TI x CTA_TJ rows, one per CTA (kSorHypCol); else the tile list, then
+// tiles of 4 x 8 rows, one per warp (kSorHyp)
 constexpr int CTA_TI = 16, CTA_TJ = 8;
 template <int G>
 int sweepHyp(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3], const double *wDev,
@@ -1132,30 +1328,32 @@ int sweepHyp(double *A, const long st[3], const long ext[3], const long lo[3], c
     char *base = (char *)scratch;
     unsigned *counter = (unsigned *)base;
     int *flags = (int *)(base + sc.flagsOff);
-    unsigned long long *table = (unsigned long long *)(base + sc.tableOff);
-    double *carry = (double *)(base + sc.carryOff);
-    if (cudaMemsetAsync(scratch, 0, sc.tableOff, s) != cudaSuccess) return -1;
-    kHypTable<G><<<(unsigned)g.nlev, 256, 0, s>>>(g, table);
-    long grid;
     if (cta) {
-        using H = HypC<G, CTA_TI, CTA_TJ>;
+        constexpr int WI = CTA_TI / TI;
+        using H = HypCol<G, WI>;
+        const long ncols = g.na * g.nb;  // a progress word each (of the scratch, sized for one flag per tile)
+        if (cudaMemsetAsync(scratch, 0, sc.flagsOff + sizeof(int) * (size_t)ncols, s) != cudaSuccess) return -1;
         static std::atomic<int> occCache[gbdev::MAX_DEVICES];
-        const int occ = gbdev::residentCtas(occCache, kSorHypCta<G, CTA_TI, CTA_TJ>, H::NTc, H::SMEM);
-        grid = (long)occ * gbdev::smCount();  // all CTAs resident at once: waits always resolve
-        if (grid > g.ntiles) grid = g.ntiles;
-        kSorHypCta<G, CTA_TI, CTA_TJ><<<(unsigned)grid, H::NTc, H::SMEM, s>>>(A, g, wDev, flags, counter, table,
-                                                                             carry, items, status, bound);
+        const int occ = gbdev::residentCtas(occCache, kSorHypCol<G, WI>, H::NTc, H::SMEM);
+        long grid = (long)occ * gbdev::smCount();  // all CTAs resident at once: waits always resolve
+        if (grid > ncols) grid = ncols;
+        kSorHypCol<G, WI><<<(unsigned)grid, H::NTc, H::SMEM, s>>>(A, g, wDev, flags, counter, items, status, bound);
+        dvmhgb_count_launches(1);
     } else {
         using H = Hyp<G>;
+        unsigned long long *table = (unsigned long long *)(base + sc.tableOff);
+        double *carry = (double *)(base + sc.carryOff);
+        if (cudaMemsetAsync(scratch, 0, sc.tableOff, s) != cudaSuccess) return -1;
+        kHypTable<G><<<(unsigned)g.nlev, 256, 0, s>>>(g, table);
         static std::atomic<int> occCache[gbdev::MAX_DEVICES];
         const int occ = gbdev::residentCtas(occCache, kSorHyp<G>, NT, H::SMEM);
-        grid = (long)occ * gbdev::smCount();
+        long grid = (long)occ * gbdev::smCount();
         const long gridCap = (g.ntiles + WPB - 1) / WPB;
         if (grid > gridCap) grid = gridCap;
         kSorHyp<G><<<(unsigned)grid, NT, H::SMEM, s>>>(A, g, wDev, flags, counter, table, carry, items, status,
                                                         bound);
+        dvmhgb_count_launches(2);
     }
-    dvmhgb_count_launches(2);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -64,7 +64,7 @@ SF_HD float ffrom(uint32_t b) {
 #endif
 }
 
-// ---- one value (host)
+// ---- one value
 #ifndef __CUDA_ARCH__
 struct Rz {  // rounding towards zero for a scope
     Rz() { fesetround(FE_TOWARDZERO); }
@@ -82,13 +82,22 @@ static inline float vmul_rz(float a, float b) {
     volatile float x = a, y = b, r = x * y;
     return r;
 }
-static inline float vpow2(float a) { return ffrom(fbits(a) & EXPMASK); }
+#else
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vfma_rz(float a, float b, float c) { return __fmaf_rz(a, b, c); }
+__device__ __forceinline__ float vmul_rz(float a, float b) { return __fmul_rz(a, b); }
 #endif
+SF_HD float vpow2(float a) { return ffrom(fbits(a) & EXPMASK); }
 template <typename V>
 struct Const;
 template <>
 struct Const<float> {
-    SF_HD float of(float c) { return c; }
+#ifdef __CUDACC__
+    static __host__ __device__ __forceinline__ float of(float c) { return c; }
+#else
+    static float of(float c) { return c; }
+#endif
 };
 
 // ---- two values in one 64-bit register (device)
@@ -245,22 +254,38 @@ FX_FN Limbs<V> unbias(V h, V m, V l) {
     return {vfma(h, Const<V>::of(2.0f), Const<V>::of(-0x1p34f)), vadd(m, c), vadd(l, c)};
 }
 
-// the double of a quotient's (or sum's) limbs, times 2^-shift: hm, mm, l and b of one cell; the value is at least 2^52 u
-SF_HD double assemble(float hm, float mm, float l, float b, int E, int shift = 0) {
+// a double from h's part of its high word, 2^23 + M, l and b, times 2^-shift
+SF_HD double assembleAt(uint32_t hw, float mm, float l, float b, int E, int shift) {
     const uint32_t il = fbits(l + 0x1p23f) & 0x7FFFFFu;
     // M 2^20 + L; the float's exponent bits (0x4B0 << 20) leave with the addend
     const uint64_t u = (uint64_t)fbits(mm) * (1u << 20) + (((uint64_t)(0u - 0x4B000u) << 32) | il);
-    const uint32_t uh = fbits(hm) * 256u + sf::hi32(u);
+    const uint32_t uh = hw + sf::hi32(u);
     const uint32_t f = (fbits(b) >> 23) + 10u;  // p - 52 modulo 32: the zero bits below the significand
 #ifdef __CUDA_ARCH__
     const uint32_t lo = __funnelshift_r((uint32_t)u, uh, f), hi = __funnelshift_r(uh, 0u, f);
 #else
     const uint32_t lo = sf::fshr((uint32_t)u, uh, f & 31u), hi = uh >> (f & 31u);
 #endif
-    // the significand's leading one adds 1 to the exponent field
+    // the significand's leading one adds 1 to the exponent field (2 where the rounding of l carried out of it)
     const uint32_t res = f * (1u << 20) + hi + ((uint32_t)(E - 161 - shift) << 20);
     return sf::from(((uint64_t)res << 32) | lo);
 }
+
+// the double of a quotient's (or sum's) limbs, times 2^-shift: hm, mm, l and b of one cell; the value is at least 2^52 u
+SF_HD double assemble(float hm, float mm, float l, float b, int E, int shift = 0) {
+    return assembleAt(fbits(hm) * 256u, mm, l, b, E, shift);
+}
+
+// RN(s) of one cell's sum of up to six values, not rounded yet (H may exceed 2^23: its low bit goes to M); s >= 2^52 u
+SF_HD double sumDouble(const Limbs<float> &s, int E) {
+    const float b = vpow2(magnitude(s));
+    const float h2 = vfma_rz(s.h, 0x1p-12f, 0x1p23f);                             // 2^23 + floor(H / 2)
+    const float odd = vfma(vadd(h2, -0x1p23f), -0x1p12f, s.h);                    // 2^11 (H mod 2)
+    const float mm = vadd(vfma(odd, 0x1p9f, s.m), 0x1p23f);
+    return assembleAt(fbits(h2) * 512u, mm, vsub(vadd(s.l, b), b), b, E, 0);
+}
+// magnitude(s) below this: s is below 2^52 u
+constexpr float SMALL1 = 0x1p23f;
 
 // RN(i u) for an integer |i| < 2^63: normalised to bit 62, its last ten bits rounded to nearest even, +0 for 0
 SF_HD double round63(int64_t i, int E) {

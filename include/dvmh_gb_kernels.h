@@ -115,8 +115,8 @@ int dvmhgb_jac2d_fused(double *A, const double *B, double *Bnew, const long st[2
  * wavefront of 4 x 8 x TK tiles, TK = 32, 16, 8 for variant 0, 1, 2, or
  * (variant 3) as 4 x 8-row columns streamed along k by one warp each, or
  * (variants 4, 5) as tiles cut along the hyperplanes i + j + k, 8
- * hyperplanes each, of 4 x 8 rows per warp (4) or 16 x 8 rows per CTA (5)
- * (a first launch lists the tiles); items = canonical partials of SUM
+ * hyperplanes each: of 4 x 8 rows, one per warp (4; a first launch lists the
+ * tiles), or columns of tiles of 16 x 8 rows walked by one CTA each (5); items = canonical partials of SUM
  * (nv-old)^2, one per row and TK-wide part of each 64-wide chunk (row, chunk,
  * part order; TK = 8 for variants 4, 5; one per row and chunk for variant 3);
  * wDev = device address of omega; scratch = dvmhgb_sor3d_scratch_bytes()
@@ -128,12 +128,12 @@ long dvmhgb_sor3d_scratch_bytes(const long lo[3], const long hi[3], int variant)
 int dvmhgb_sor3d_sweep(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3],
                        const double *wDev, double *items, void *scratch, int *status, int variant, void *stream);
 /* The same sweep with its bounded waits made explicit.  Every wait for a
- * predecessor tile (column, variant 3) polls at most pollLimit times
+ * predecessor tile (column, variants 3 and 5) polls at most pollLimit times
  * (dvmhgb_sor3d_sweep: 2^24, about 1-4 s) before the kernel writes its timeout
  * code 0x50520001 to *status, sets the top bit of the hand-out counter (the
  * first word of scratch) so that no warp takes another tile, and returns; the
  * runtime reports a non-zero status word at its next synchronisation (exit
- * status 1).  firstIndex > 0 starts the hand-out at that tile: the tiles
+ * status 1).  firstIndex > 0 starts the hand-out at that tile (column): the tiles
  * before it are left to nobody, so their successors' waits run out -- how the
  * tests make a wait expire without a fault.  -1 for pollLimit < 1 or a
  * negative firstIndex. */
