@@ -172,6 +172,14 @@ struct Var : Obj {
     bool hostActual = true, devActual = false;
     std::string name;
     DvmType hdr[4] = {};  // its rank-0 header (dvmh_variable_gen_header_C with rank 0): hdr[0] = this
+    // Reduction results reach the host without a copy of their own: a fold writes them to the device copy and to a
+    // mirror of it in pinned host memory.  written[g] == epoch: 4-byte granule g of the mirror holds what the device
+    // copy holds, since an upload or a handler that asked for the device address last made the mirror worthless.
+    char *mirror = nullptr;
+    std::vector<uint32_t> written;
+    uint32_t epoch = 1;
+    size_t current = 0;    // granules of this epoch
+    bool exposed = false;  // kernels may write the device copy directly: the mirror is never read
 };
 
 // An array declared without its size (dvmh_array_declare_C); dvmh_array_alloc_C
@@ -311,8 +319,13 @@ void copyBoxD2H(Array *a, const long lo[], const long hi[]);
 void streamSync();
 
 // reduction fold (canonical tree) writing the final value to dst / dstLoc
+// dst, loc and their pinned mirrors (null: none)
+struct FoldDst {
+    void *dst, *loc;
+    void *mirror, *mirrorLoc;
+};
 void launchRedFold(int op, int vtype, long count, long elemCount, const void *items, const void *locItems,
-                   long locSize, void *dst, void *dstLoc, cudaStream_t s, std::vector<void *> &scratch);
+                   long locSize, const FoldDst &to, cudaStream_t s, std::vector<void *> &scratch);
 void fillIdentity(int op, int vtype, void *items, long n, cudaStream_t s);
 // one deferred reduction fold (batched handlers): FP64, one element
 struct FoldJob {
@@ -320,7 +333,7 @@ struct FoldJob {
     long count;
     const void *items, *locItems;
     long locSize;
-    void *dst, *dstLoc;
+    FoldDst to;
     long blockBase;  // first of this job's 2048-item spans in the batch (set by launchRedFoldBatch)
 };
 bool foldBatchable(int op, int vtype, long count, long elemCount);
@@ -350,6 +363,8 @@ void ensureHostActual(Array *a);
 void ensureVarDev(Var *v);
 void varH2D(Var *v);
 void varD2H(Var *v);
+void varMirror(Var *v);                                 // give a reduction variable its mirror, if it can have one
+void varMirrored(Var *v, size_t off, size_t len);       // a launched fold writes these bytes of both copies
 void varForgetStaging(const Var *v);  // the variable is dropped: its pinned staging buffer too
 void fillDesc(Array *a);
 size_t maxDeviceElems();  // the most device elements of any live array with a device copy

@@ -238,6 +238,8 @@ Var *varGet(const void *addr, size_t size) {
             dropOverlaps(v->addr + v->size, hi, v);
             if (v->dev) devFree(v->dev);
             v->dev = nullptr;
+            v->mirror = nullptr;
+            v->written.clear();
             v->size = size;
             v->devActual = false;
             v->hostActual = true;
@@ -624,6 +626,7 @@ void *dvmh_get_device_addr_C(DvmType deviceNum, const void *addr) {
     size_t off = 0;
     Var *v = varAt(addr, &off);
     GB_CHECK(v && v->dev, "can not get the device address of a variable unknown to the region");
+    v->exposed = true;
     return v->dev + off;
 }
 

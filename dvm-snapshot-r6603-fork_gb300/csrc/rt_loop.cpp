@@ -107,6 +107,10 @@ struct LayoutState {
     }
 };
 
+struct MirrorWrite {
+    Var *var;
+    size_t off, len;
+};
 struct CachedGraph {
     uint64_t key;
     std::vector<uint64_t> sig;
@@ -117,6 +121,7 @@ struct CachedGraph {
     std::vector<void *> hostScratch;
     std::vector<Array *> swaps;
     std::vector<std::pair<Array *, LayoutState>> layouts;  // layout changes, in order
+    std::vector<MirrorWrite> mirrors;                      // what its folds write to variables' mirrors
     long launches = 0;
 };
 static std::list<CachedGraph> graphCache;  // most recently used first
@@ -173,6 +178,7 @@ struct ExecCtx {
     std::vector<void *> *keepHost = nullptr;  // pinned host scratch kept with it
     std::vector<Array *> *swaps = nullptr;    // swaps performed (recorded for replays)
     std::vector<std::pair<Array *, LayoutState>> *layouts = nullptr;  // layout changes, likewise
+    std::vector<MirrorWrite> *mirrors = nullptr;                      // writes to variables' mirrors, likewise
 };
 static ExecCtx ctx;
 
@@ -468,6 +474,8 @@ static std::vector<uint64_t> signature(const std::vector<Loop *> &q) {
             sigAdd(s, (uint64_t)r.locVar);
             sigAdd(s, (uint64_t)(r.var ? r.var->dev : nullptr));
             sigAdd(s, (uint64_t)(r.locVar ? r.locVar->dev : nullptr));
+            sigAdd(s, (uint64_t)(r.var ? r.var->mirror : nullptr));
+            sigAdd(s, (uint64_t)(r.locVar ? r.locVar->mirror : nullptr));
         }
     }
     sigAdd(s, (uint64_t)settings.fuse);
@@ -578,6 +586,7 @@ static void queueFlushPrefix(size_t count) {
             launchGraph(*it);
             for (Array *a : it->swaps) std::swap(a->dev, a->devAlt);
             for (auto &pl : it->layouts) pl.second.applyTo(pl.first);
+            for (auto &m : it->mirrors) varMirrored(m.var, m.off, m.len);
             stats.graph_replays++;
             stats.kernel_launches += it->launches;
             graphCache.splice(graphCache.begin(), graphCache, it);
@@ -596,6 +605,7 @@ static void queueFlushPrefix(size_t count) {
     ctx.keepHost = &g.hostScratch;
     ctx.swaps = &g.swaps;
     ctx.layouts = &g.layouts;
+    ctx.mirrors = &g.mirrors;
     GB_CUDA(cudaStreamBeginCapture(gpu.stream, cudaStreamCaptureModeRelaxed));
     runQueued(q);
     cudaGraph_t graph = nullptr;
@@ -770,6 +780,7 @@ void dvmh_loop_reduction_C(DvmType curLoop, DvmType redType, void *arrayAddr, Dv
     r.var = v;
     r.varOff = off;
     ensureVarDev(v);
+    varMirror(v);
     if (!v->devActual || (v->hostActual && !varInRegion(v))) {
         varH2D(v);
         v->devActual = true;
@@ -784,6 +795,7 @@ void dvmh_loop_reduction_C(DvmType curLoop, DvmType redType, void *arrayAddr, Dv
         r.locVar = lv;
         r.locVarOff = loff;
         ensureVarDev(lv);
+        varMirror(lv);
         if (!lv->devActual || (lv->hostActual && !varInRegion(lv))) {
             varH2D(lv);
             lv->devActual = true;
@@ -1107,19 +1119,30 @@ void dvmh_loop_cuda_red_prepare_C(DvmType curLoop, DvmType redIndex, DvmType cou
     }
 }
 
+// the mirror of the fold's result, if the variable has one: written with the result, now and by every replay
+static void mirrorFold(Var *v, size_t off, size_t len, void **mirror) {
+    if (!v->mirror || v->exposed) return;
+    *mirror = v->mirror + off;
+    varMirrored(v, off, len);
+    if (ctx.mirrors) ctx.mirrors->push_back({v, off, len});
+}
+
 void dvmh_loop_cuda_red_finish_C(DvmType curLoop, DvmType redIndex) {
     SpecLoop *s = specOf(curLoop, "dvmh_loop_cuda_red_finish");
     CudaRed &cr = cudaRed(s, redIndex, "dvmh_loop_cuda_red_finish");
     GB_CHECK(cr.items, "reduction #%ld finished before dvmh_loop_cuda_red_prepare_C", (long)redIndex);
     GB_CHECK(!cr.finished, "reduction #%ld finished twice", (long)redIndex);
     Reduction &r = s->loop->reds[redIndex - 1];
-    char *dst = r.var->dev + r.varOff;
-    char *dstLoc = r.locVar ? r.locVar->dev + r.locVarOff : nullptr;
+    FoldDst to = {r.var->dev + r.varOff, nullptr, nullptr, nullptr};
+    mirrorFold(r.var, r.varOff, (size_t)(r.esize * r.count), &to.mirror);
+    if (r.locVar) {
+        to.loc = r.locVar->dev + r.locVarOff;
+        mirrorFold(r.locVar, r.locVarOff, (size_t)(r.locSize * r.count), &to.mirrorLoc);
+    }
     if (deferFolds && foldBatchable(r.op, r.vtype, cr.count, r.count))
-        deferred.push_back({r.op, cr.count, cr.items, cr.locItems, r.locSize, dst, dstLoc});
+        deferred.push_back({r.op, cr.count, cr.items, cr.locItems, r.locSize, to, 0});
     else
-        launchRedFold(r.op, r.vtype, cr.count, r.count, cr.items, cr.locItems, r.locSize, dst, dstLoc, s->stream,
-                      s->scratch);
+        launchRedFold(r.op, r.vtype, cr.count, r.count, cr.items, cr.locItems, r.locSize, to, s->stream, s->scratch);
     cr.finished = true;
 }
 
