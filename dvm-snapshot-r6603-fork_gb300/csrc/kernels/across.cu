@@ -1002,6 +1002,7 @@ __global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g
     extern __shared__ double sm[];  // box [TI WI + 2][RS], then squares and nodes [SQS][NTc]
     __shared__ long sIdx;
     __shared__ bool sAhead[2];
+    gbdev::nextMayLaunch();
     const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5, li = lane / TJ, lj = lane % TJ;
     const int lr = li, lp = lj;     // staging: a lane copies position lp of rows lr, lr + 4, ...
     double *box = sm + wi * TI * RS;                   // the warp's rows and their faces

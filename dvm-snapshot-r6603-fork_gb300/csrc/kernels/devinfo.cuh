@@ -9,6 +9,28 @@
 
 namespace gbdev {
 
+// Programmatic stream serialisation: a kernel launched by launchAfter() may start as soon as every CTA of the kernel
+// before it has called nextMayLaunch() or ended.  waitForKernelBefore() waits until that kernel (and what it waited
+// for) has ended and its writes are visible; every thread of a kernel so launched calls it, before it reads anything
+// that kernel writes, and before it ends.
+__device__ __forceinline__ void nextMayLaunch() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void waitForKernelBefore() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline cudaError_t launchAfter(void (*kernel)(Params...), unsigned blocks, unsigned threads, cudaStream_t s,
+                               Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.stream = s;
+    c.attrs = &attr;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, Params(args)...);
+}
+
 constexpr int MAX_DEVICES = 64;
 
 // the current device's ordinal, or -1

@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(256, 2)
                int nitems, int rowsToo) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double shr[8];
+    if (FUSED) gbdev::nextMayLaunch();
     const int lane = threadIdx.x & 31;
     const long strip = blockIdx.x * 8L + (threadIdx.x >> 5);
     uint64_t mb = 0;

@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     using fx::f32x2;
     using Limbs = fx::Limbs<f32x2>;
     extern __shared__ unsigned char dyn[];
+    if (U) gbdev::nextMayLaunch();
     unsigned char *base = dyn + ((128u - (tma::smemAddr(dyn) & 127u)) & 127u);
     float *ring = reinterpret_cast<float *>(base + NS * SLOT);
     uint64_t *bars = reinterpret_cast<uint64_t *>(base + NS * SLOT + limb::ringOf(JT));
