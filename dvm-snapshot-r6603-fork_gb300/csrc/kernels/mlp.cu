@@ -38,7 +38,8 @@ constexpr long OFF_W1 = 0, OFF_B1 = OFF_W1 + (long)H * D, OFF_W2 = OFF_B1 + H, O
 // gradients: 16 CTAs, each a serial pass over all rows.  Row ranges per CTA give every SM a share of that
 // contraction.  A warp multiplies 5 rows by 64 columns (2 a lane): 13 shared-memory cycles per 10 of FMAs, against
 // 24 per 8 for 2 rows by 128 columns; 40 rows a tile is one tile per CTA where the partials allow 38.6 rows a CTA.
-// Loss, gradient and Adam step on 4096 rows, back to back: 830 us before, 62 with 2 rows by 128 columns, 40 now.
+// Loss, gradient and Adam step on 4096 rows, back to back: 830 us before, 62 with 2 rows by 128 columns, 40 with 5
+// by 64, 37 since the fold and Adam are launched while the kernel before them runs.
 constexpr int MT = 512;       // threads of a CTA: 16 warps, warps 2g and 2g + 1 on rows 5g .. 5g + 4 of a tile
 constexpr int WR = 5, MR = 8 * WR;
 constexpr int XP = D + 2;     // row stride of the staged features
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(MT, 1)
          float *pred, float *out, long pitch, float *lossOut) {
     extern __shared__ __align__(16) float sm[];
     float *W1t = sm, *W2t = W1t + D * HP, *Xs = W2t + H * HP, *H1 = Xs + MR * XP, *ps = H1 + MR * H;
+    gbdev::nextMayLaunch();
     float *W2 = ps + 2 * MR, *Z2 = W2 + H * H, *Z1 = Z2 + MR * H, *es = Z1 + MR * H;
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 6, half = (tid >> 5) & 1;
     const int row0 = WR * group, col0 = 64 * half + 2 * lane;
@@ -224,6 +226,8 @@ __global__ void __launch_bounds__(256) kGradFold(const float *__restrict__ part,
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const long p = blockIdx.x * 32L + tx;
     float s = 0;
+    gbdev::nextMayLaunch();
+    gbdev::waitForKernelBefore();
     if (p <= NPARAM) {
 #pragma unroll 4
         for (int c = ty; c < ctas; c += 8) s += part[c * pitch + p];
@@ -253,6 +257,7 @@ bool mlpShared() {  // raised once per device
 
 __global__ void kAdam(float *p, const float *g, float *m, float *v, long cnt, float lr, float b1, float b2, float eps,
                       float c1, float c2) {
+    gbdev::waitForKernelBefore();
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < cnt; i += (long)gridDim.x * blockDim.x) {
         float mi = b1 * m[i] + (1 - b1) * g[i];
         float vi = b2 * v[i] + (1 - b2) * g[i] * g[i];
@@ -311,7 +316,9 @@ int dvmhgb_mlp_loss_grad(const float *P, const float *X, const float *y, long n,
     const long ctas = room < 1 ? 1 : (room < gbdev::smCount() ? room : gbdev::smCount());
     const long per = rowsPerCta(n, ctas), grid = (n + per - 1) / per;
     kMlp<true><<<(unsigned)grid, MT, MLP_SMEM, s>>>(P, X, y, n, per, nullptr, grid > 1 ? work : grad, pitch, loss);
-    if (grid > 1) kGradFold<<<(unsigned)((pitch + 31) / 32), 256, 0, s>>>(work, (int)grid, pitch, n, grad, loss);
+    if (grid > 1 && gbdev::launchAfter(kGradFold, (unsigned)((pitch + 31) / 32), 256, s, work, (int)grid, pitch, n, grad,
+                                       loss) != cudaSuccess)
+        return -1;
     dvmhgb_count_launches(grid > 1 ? 2 : 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -320,7 +327,9 @@ int dvmhgb_mlp_adam(float *P, const float *grad, float *m, float *v, long step, 
     if (!P || !grad || !m || !v || step < 1) return -1;
     const float b1 = 0.9f, b2 = 0.999f;
     float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-    kAdam<<<64, 256, 0, (cudaStream_t)stream>>>(P, grad, m, v, NPARAM, lr, b1, b2, 1e-8f, c1, c2);
+    if (gbdev::launchAfter(kAdam, 64, 256, (cudaStream_t)stream, P, grad, m, v, NPARAM, lr, b1, b2, 1e-8f, c1, c2) !=
+        cudaSuccess)
+        return -1;
     dvmhgb_count_launches(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
