@@ -24,7 +24,7 @@
 // the pair: the update kernel, then that stencil in place
 #define DEF_FUSED 25
 // a step's stencil with the next step's update in one pass (the pairing the runtime forms across steps)
-#define DEF_STNUPD 5  // 0.72 (the q61 pass it replaced: 1.09)
+#define DEF_STNUPD 4  // 0.677 a step (variant 5: 0.707; the q61 pass these replaced: 1.09)
 
 namespace {
 
