@@ -22,7 +22,7 @@ Printed as one JSON line:
              over the timed region, against the measured HBM copy bandwidth
   roofline_fp64  the stencil's 5 FP64 additions per cell as if all ran on the
              FP64 unit, against that unit's measured addition rate: a fraction
-             above 1 is work moved to the integer pipes (q61 fixed point)
+             above 1 is work moved to the FP32 pipe (exact limb arithmetic)
   cpu_baseline  the CPU port of the same loops (oracle/restate.c, OpenMP,
              static schedule over the outermost loop like the reference host
              handlers) on this machine's host cores, bounded sample
@@ -49,7 +49,7 @@ sys.path.insert(0, ROOT)
 N_DEFAULT = 512
 SEED = 20261203
 BYTES_PER_CELL = 32  # A and B each read once and written once per step
-FP64_ADDS_PER_CELL = 5  # the stencil's additions (mostly in q61 fixed point on the integer pipes)
+FP64_ADDS_PER_CELL = 5  # the stencil's additions (on FP32 limbs)
 
 
 def peaks():
@@ -306,18 +306,18 @@ def main():
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": None,
                          "kernel": (pair + ": a step's stencil with the next step's update in one pass -- "
-                                    "kStencil3T<3> (planes staged by TMA, q61 sums on the integer pipes, |B - A| on "
-                                    "the FP64 unit, B and the new A written) -- in the step's captured graph")
+                                    "kStencil3L<3> (planes staged by TMA, sums and |B - A| on FP32 limbs, B and the "
+                                    "new A written) -- in the step's captured graph")
                                    if pair == "loop_jac3d_stnupd_cuda" else
                                    (pair + ": the update+stencil pair of the fusion rule -- kUpdate (fixed-point "
-                                    "MAX, A = B), then kStencil3T writing B in place -- in the step's captured graph"),
+                                    "MAX, A = B), then kStencil3L writing B in place -- in the step's captured graph"),
                          "bytes_per_launch": BYTES_PER_CELL * cells, "launch_ms": kern_ms,
                          "hbm_frac_of_step": BYTES_PER_CELL * cells / (ms * 1e-3) / 1e9 / peak},
             "roofline_fp64": {"bound": "fp64", "achieved": fp64_achieved, "peak": fp64_peak, "unit": "FP64 add/s",
                               "frac": fp64_achieved / fp64_peak if fp64_peak else None,
                               "ops_per_cell": FP64_ADDS_PER_CELL,
                               "peak_kind": "measured (dvmhgb_fp64_add_rate: independent DADD chains on every SM)",
-                              "note": "FP64-add equivalent: most additions run as q61 integer additions"},
+                              "note": "FP64-add equivalent: the additions run on FP32 limbs"},
             "clocks": ck, "e2e": e2e, "gpu_launches": st["kernel_launches"]}
     traffic = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(traffic):

@@ -3,7 +3,7 @@
 //   dst[i][j] = src[i][j] + c * (src[i-1][j] + src[i+1][j] + src[i][j-1] + src[i][j+1] - 4.0 * src[i][j])
 //   sum += dst[i][j];  if (dst[i][j] < mn) { mn = dst[i][j]; loc = {i, j}; }
 //
-// A warp walks a strip: up to DVMHGB_HEAT_STRIP consecutive rows of one
+// A warp walks a strip: up to DVMHGB_HEAT_ROWS(variant) consecutive rows of one
 // 64-wide chunk of j aligned to a multiple of 64 of the array index (lane l
 // holds j = base+2l, base+2l+1 as one 128-bit access).  Rows i-1, i, i+1 roll
 // through registers with row i+2 in flight, so every source row is read once
