@@ -936,14 +936,15 @@ __global__ void __launch_bounds__(NT) kSorHyp(double *A, HGeo g, const double *w
 // of the tile before) sums on the FP64 unit; after a tile with three such steps, or with negative values, the next eight
 // tiles do.
 //
-// What bounds it: the chain of tile planes a + b + c (52 for 97^3, 214 for 384^3) at about 11,000 cycles each: 8 steps
-// of 870 - 950 (the dependent chain of split, five additions, assembly, two FP64 operations and the barrier), 700 for
-// the faces, 1,100 to store and publish, 1,000 until the next column sees it.  Measured per sweep (values in one
-// range), against tiles of one warp (variant 4) and one tile of 16 x 8 rows per CTA and hand-out, with all sums on
-// FP64: 97^3 295 us (366, 316), 384^3 1770 us (2035, 2037).  With signed values: 97^3 322 us (365), 384^3 2250 us (2035):
-// variant 4 remains for large boxes of those.  What did not help: limbs kept in shared memory and split once by their
-// producer (unrolled or not, 288 and 1788 us), four CTAs per SM (1946 us at 384^3), 32 x 8 rows (2166 us), 8 x 8 (1749
-// us; 320 us at 97^3), unrolled steps (instruction cache: 1821 - 1880 us).
+// What bounds it: the chain of tile planes a + b + c (52 for 97^3, 214 for 384^3) at about 10,500 cycles each: 8 steps
+// of 740 - 950 (the dependent chain of split, five additions, assembly, two FP64 operations and the barrier), 700 for
+// the faces, 500 to publish, 1,000 until the next column sees it.  Measured per sweep (values in one range), against
+// tiles of one warp (variant 4) and one tile of 16 x 8 rows per CTA and hand-out, with all sums on FP64: 97^3 269 us
+// (366, 316), 384^3 1690 us (2035, 2037).  With signed values: 97^3 300 us (365), 384^3 2175 us (2035): variant 4 remains
+// for large boxes of those.  Storing the last rows in the steps and publishing from another warp than the one that
+// polls, instead of a store phase, a barrier and warp 0 for both: 281 -> 269, 1747 -> 1690.  What did not help: limbs
+// kept in shared memory and split once by their producer (unrolled or not, 288 and 1788 us), four CTAs per SM (1946 us
+// at 384^3), 32 x 8 rows (2166 us), 8 x 8 (1749 us; 320 us at 97^3), unrolled steps (instruction cache: 1821 - 1880 us).
 
 template <int G, int WI>
 struct HypCol {
@@ -1002,6 +1003,8 @@ __global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g
     extern __shared__ double sm[];  // box [TI WI + 2][RS], then squares and nodes [SQS][NTc]
     __shared__ long sIdx;
     __shared__ bool sAhead[2];
+    // warps with other things to do neither poll (warp 0 loads the -i face) nor publish and poll at once
+    constexpr int POLL = 32 * (WI / 2), PUBLISH = NTc - 1;
     gbdev::nextMayLaunch();
     const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5, li = lane / TJ, lj = lane % TJ;
     const int lr = li, lp = lj;     // staging: a lane copies position lp of rows lr, lr + 4, ...
@@ -1029,9 +1032,9 @@ __global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g
         const long a = (sd - (g.nb - 1) > 0 ? sd - (g.nb - 1) : 0) + idx - columnsBefore(sd, g.na, g.nb), b = sd - a;
         const long ra = TI * (WI * a + wi), rb = TJ * b;  // the warp's first row
         const int cmin = (int)hypCmin<G>(g, a, b), cmax = (int)hypCmax<G>(g, a, b);
-        // thread 0 waits for column (a-1, b), thread 1 for (a, b-1)
-        const bool waits = tid == 0 ? a > 0 : tid == 1 && b > 0;
-        const long pa = a - (tid == 0), pb = b - (tid == 1);
+        // thread POLL waits for column (a-1, b), the next one for (a, b-1)
+        const bool waits = tid == POLL ? a > 0 : tid == POLL + 1 && b > 0;
+        const long pa = a - (tid == POLL), pb = b - (tid == POLL + 1);
         const int *before = prog + pa * g.nb + pb;
         const int plast = waits ? (int)hypCmax<G>(g, pa, pb) : 0;
         int seen = 0;
@@ -1135,11 +1138,14 @@ __global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g
             }
             box[(1 + lr) * RS + at + lp] = f2;
             copiesDone();
-            if (tid < 2) sAhead[tid] = !waits || seen > (c + 1 < plast ? c + 1 : plast);
+            if (tid == POLL || tid == POLL + 1) sAhead[tid - POLL] = !waits || seen > (c + 1 < plast ? c + 1 : plast);
             __syncthreads();
             // the next tile's faces already: the columns before this one are further ahead
             ahead = c < cmax && sAhead[0] && sAhead[1];
             if (ahead) faces(c + 1);
+            // what the next columns read, the CTA's last rows along i and j, is stored as it is computed
+            const bool last = (wi == WI - 1 && li == TI - 1) || lj == TJ - 1;
+            double *cell = A + i * g.s0 + j * g.s1 + g.lo2 + rk0;
             // 2. the dependent chain: G steps, every lane on its own row.  The terms that do not depend on the step
             //    before (+i, +j, +k of the next step, the part the last tile closed) fill the FP64 unit's latencies
             big = 0;
@@ -1185,7 +1191,10 @@ __global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g
                 const double nv = cold + c2 * s;
                 const double kn = x[p2];
                 if (LIMB) terms(p2, kn);
-                if (act) x[p0] = nv;
+                if (act) {
+                    x[p0] = nv;
+                    if (last) cell[t] = nv;
+                }
                 __syncthreads();
                 dv = nv - old;
                 actd = act;
@@ -1203,27 +1212,16 @@ __global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g
 #pragma unroll 1
                 for (int t = 0; t < G; t++) step(t, std::true_type());
             }
-            // 3. store what the successors read -- the rows li = 3 and lj = 7 -- and publish the tile, then store its
-            //    other cells (read by no other column of this sweep)
+            // 3. publish the tile: the last step's barrier orders every thread's stores of its last rows before this
+            //    release at GPU scope, which publishes them (release cumulativity) without a sequentially consistent
+            //    fence in every thread.  Then store the other cells (read by no other column of this sweep)
             auto store = [&](int qi, int qj) {  // 4 rows x 8 positions
                 if ((qj ? inJ4 : inJ0) && qi < rowsS && (unsigned)(c * G + q0 - qi - qj) < (unsigned)nk)
                     *(src + c * G + qi * (g.s0 - 1) + qj * (g.s1 - 1)) =
                         box[(1 + qi) * RS + (1 + qj + lr) * SKP + at + lp];
             };
+            if (tid == PUBLISH) stRelease(prog + a * g.nb + b, c + 1);
             const bool edge = wi == WI - 1;  // the warp with the tile's last row
-            if (edge) {
-                store(TI - 1, 0);
-                store(TI - 1, 4);
-            }
-            if (lr == 3) {
-#pragma unroll
-                for (int qi = 0; qi < TI; qi++)
-                    if (qi < TI - 1 || !edge) store(qi, 4);
-            }
-            // the barrier orders every thread's stores before thread 0's release at GPU scope, which publishes
-            // them (release cumulativity) without a sequentially consistent fence in every thread
-            __syncthreads();
-            if (tid == 0) stRelease(prog + a * g.nb + b, c + 1);
 #pragma unroll
             for (int qi = 0; qi < TI; qi++)
                 if (qi < TI - 1 || !edge) {
