@@ -1193,10 +1193,11 @@ int launchSU(const double *A, double *B, double *Aalt, const Box3 &b, const long
 
 // (rows per thread, plane slots, CTAs per SM) of the limb kernels' variants: the stencil's 22 + v (v < 5) and the
 // cross-step pass's v.  At 512^3, us (stencil a call / a batched step of the cross-step pass with the faces' copy beside
-// it and the fold): 0: 703 / 830, 1: 620 / 722, 2: 617 / 686, 3 and 5: 612 / 707, 4: 616 / 677.  Two rows a thread take
-// a quarter fewer instructions per cell and hold half the warps: the faster ones where the pass also takes |B - A| and
-// writes twice, and with registers left on the SM for the copy's CTAs; 256^3: 116 against 121, 130^3: 40 against 41.5.
-#define DVMHGB_LIMB_SHAPES(C) C(0, 1, 5, 4) C(1, 1, 5, 3) C(2, 2, 5, 2) C(3, 1, 6, 3) C(4, 2, 6, 2) C(5, 1, 6, 3)
+// it and the fold): 0: 703 / 830, 1: 620 / 722, 2: 617 / 686, 3 and 5: 612 / 707, 4: 616 / 673 (six slots 678, seven
+// 706, four 746; three rows a thread at one CTA 873).  Two rows a thread take a quarter fewer instructions per cell and
+// hold half the warps: the faster ones where the pass also takes |B - A| and writes twice, and with registers left on
+// the SM for the copy's CTAs; 256^3: 116 against 121, 130^3: 40 against 41.5.
+#define DVMHGB_LIMB_SHAPES(C) C(0, 1, 5, 4) C(1, 1, 5, 3) C(2, 2, 5, 2) C(3, 1, 6, 3) C(4, 2, 8, 2) C(5, 1, 6, 3)
 
 template <bool FUSED>
 void launch3(int variant, const St3Geom &g, double *A, const double *B, double *Out, const Box3 &b, double *items,
