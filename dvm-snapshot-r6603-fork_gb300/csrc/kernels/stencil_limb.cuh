@@ -27,6 +27,17 @@
 // from the doubles of the plane slots, bit for bit the same; so is one whose
 // quotient is too small for the assembly, by the integer division.
 //
+// Plain planes.  A plane that no range holds is done by a loop of its own, with
+// no split before it and the limbs of the next two planes made anew after it; the
+// third in a row (the first of a chunk) is followed by eight such planes, then
+// sixteen, up to sixty-four at a time.  With every plane split and looked through
+// first, and rows outside the box computed too, values in [-1, 1) took 254 us for
+// the stencil and 342 for the cross-step pass at 255^3, 1500 and 2220 at 512^3,
+// 1186 and 2790 for a box of 2000 x 2 x 2000; now 178 and 270, 1350 and 1940, 150
+// and 425 (the kernels before the limbs: 205 and 285, 1535 and 2046, 226 and 336).
+// A loop of its own also because as a branch of the step, in its three copies, it
+// took the FP64 path 2790 us at 512^3: instruction fetches.
+//
 // M = 3: the new B of a cell meets A's limbs (the plane's own) in registers, so
 // |B - A| is a difference of limbs, exact as an integer.  Only its FP32 value
 // (off by less than 2^-21 relatively) is formed for every cell; the exact
@@ -94,6 +105,9 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     // the timeout flag, one per parity of the step: set before the step's barrier, read after it
     __shared__ int stopAt[2];
     __shared__ unsigned topExp;
+    // planes that no range held: the last one's step, how many in a row (the chunk's first counts as the third), how many
+    // plain planes follow the next that is one too many
+    __shared__ int missAt, missed, nextPlain;
     __shared__ float seenMax;  // U: |B - A| (u units) some thread has entered exactly, times (1 - 2^-20)
     __shared__ double shr[TY];
 
@@ -106,8 +120,9 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     const long k = kb + 2 * lane, j = jb + JT * ty;
     const bool k0 = k >= b.lo2 && k <= b.hi2, k1 = k + 1 >= b.lo2 && k + 1 <= b.hi2;
     // the cells of the loop box: bits 0, 1 the first row's pair, bits 2, 3 the second's; U: from bit 4, the others of a
-    // row of the box, whose A carries over
-    int cells = 0;
+    // row of the box, whose A carries over; MINE: the warp has a row of the box
+    constexpr int MINE = 256;
+    int cells = j <= b.hi1 ? MINE : 0;
     float tiny[JT][2];
     f32x2 mask[JT];
 #pragma unroll
@@ -117,8 +132,8 @@ __global__ void __launch_bounds__(TX *TY, MINB)
         if (U && j + r <= b.hi1)
             cells |= (!in0 && k < b.e2 ? 16 << 2 * r : 0) | (!in1 && k + 1 < b.e2 ? 32 << 2 * r : 0);
         // a quotient below the assembly's range counts in the box only; |B - A| outside it is 0
-        tiny[r][0] = in0 ? fx::SMALL6 : 0.0f;
-        tiny[r][1] = in1 ? fx::SMALL6 : 0.0f;
+        tiny[r][0] = in0 ? fx::SMALL6 : -__builtin_huge_valf();
+        tiny[r][1] = in1 ? fx::SMALL6 : -__builtin_huge_valf();
         mask[r] = fx::pack(in0 ? 1.0f : 0.0f, in1 ? 1.0f : 0.0f);
     }
     asm volatile("" : "+r"(cells));  // kept, not computed again every step
@@ -141,15 +156,20 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     constexpr int RP = BX / 2;  // pairs of a row
     constexpr int HALO = 2 * RP + 2 * TJ;
     static_assert(HALO == CELLS / 2 - TX * TJ && HALO <= TX * TY, "own pairs, then halo pairs");
-    const int own = (JT * ty + 1) * BX + 2 + 2 * lane;
+    // (a thread whose pairs no cell of the box reads takes the CTA's first one, so that theirs do not count)
+    const int place = (JT * ty + 1) * BX + 2 + 2 * lane;
+    const int own = j <= b.hi1 + 1 && k <= b.hi2 + 1 ? place : BX + 2;
     int halo = -1;
     {
         const int h = (tid + 32 * (int)((blockIdx.x + blockIdx.y + blockIdx.z) & 7)) & (TX * TY - 1);
         if (h < RP) halo = 2 * h;
         else if (h < 2 * RP) halo = (TJ + 1) * BX + 2 * (h - RP);
         else if (h < HALO) halo = (1 + (h - 2 * RP) / 2) * BX + ((h - 2 * RP) & 1 ? BX - 2 : 0);
+        // beyond the last row and column that a cell of the box reads
+        if (halo >= 0 && (jb - 1 + halo / BX > b.hi1 + 1 || kb - 2 + halo % BX > b.hi2 + 1)) halo = -1;
     }
 
+    constexpr int MISSES = 3, PLAIN = 8, PLAIN_MAX = 64;  // (above)
     int E = fx::E_DEFAULT;  // the range's smallest exponent field
     auto splitPair = [&](const double *src, bool &ok) -> Limbs {
         const uint4 w = *reinterpret_cast<const uint4 *>(src);
@@ -166,17 +186,18 @@ __global__ void __launch_bounds__(TX *TY, MINB)
         Limbs v[JT];
         bool ok;
     };
-    auto splitOwn = [&](const double *s, Own &o) {
-        o.ok = true;
+    auto splitOwn = [&](const double *s, Own &o) -> bool {
+        bool ok = true;
 #pragma unroll
-        for (int r = 0; r < JT; r++) o.v[r] = splitPair(s + own + r * BX, o.ok);
+        for (int r = 0; r < JT; r++) o.v[r] = splitPair(s + own + r * BX, ok);
+        o.ok = ok;
+        return ok;
     };
     // a plane's limbs: the own pairs' to o and, with the halo pair's, to the ring
     auto splitPlane = [&](const double *s, float *l, Own &o) -> bool {
-        splitOwn(s, o);
+        bool ok = splitOwn(s, o);
 #pragma unroll
         for (int r = 0; r < JT; r++) limb::stLimbs(l + own + r * BX, CELLS, o.v[r]);
-        bool ok = o.ok;
         if (halo >= 0) limb::stLimbs(l + halo, CELLS, splitPair(s + halo, ok));
         return ok;
     };
@@ -198,6 +219,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
 
     if (tid == 0) {
         stopAt[0] = stopAt[1] = 0;
+        missAt = -1, missed = 2, nextPlain = PLAIN;
         seenMax = 0.0f;
         for (int s = 0; s < NS; s++) tma::mbarInit(tma::smemAddr(bars + s), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -218,10 +240,70 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     const long toOut2 = U ? (Out2 - Out) : 0;
     int t = 0;
 
-    // step t: plane c = t + 1 from planes m, c, p; false when the loop ends
+    // plane t + 1 on the FP64 unit, from the doubles of the slots
+    auto native = [&](double v[JT][2]) {
+        const double *pm = slotOf(t) + own, *pc = slotOf(t + 1) + own, *pp = next + own;
+#pragma unroll
+        for (int r = 0; r < JT; r++, pm += BX, pc += BX, pp += BX) {
+            const double2 ac = *reinterpret_cast<const double2 *>(pc);
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const double first = sf::nadd(sf::nadd(pm[e], pc[e - BX]), e ? ac.x : pc[-1]);
+                v[r][e] = sf::div3p2(sf::nadd(sf::nadd(sf::nadd(first, e ? pc[2] : ac.y), pc[e + BX]), pp[e]), 1);
+                if (U && (cells >> (2 * r + e) & 1)) mb = sf::absmax_bits(sf::nadd(v[r][e], -(e ? ac.y : ac.x)), mb);
+            }
+        }
+    };
+    auto store = [&](const double v[JT][2]) {
+#pragma unroll
+        for (int r = 0; r < JT; r++) {
+            double *o = out + r * b.s1;
+            if (__builtin_expect((cells >> 2 * r & 3) == 3, 1)) {
+                st2cs(o, make_double2(v[r][0], v[r][1]));
+                if (U) st2cs(o + toOut2, make_double2(v[r][0], v[r][1]));  // A = B into A's second buffer
+            } else {
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    if (cells >> (2 * r + e) & 1) {
+                        o[e] = v[r][e];
+                        if (U) o[toOut2 + e] = v[r][e];
+                    } else if (U && (cells >> (2 * r + e) & 16)) {
+                        o[toOut2 + e] = slotOf(t + 1)[place + r * BX + e];
+                    }
+                }
+            }
+        }
+    };
+    // to the next step; `ok` of every thread's part of plane t + 2
+    auto advance = [&](bool ok) -> bool {
+        out += b.s0;
+        next = reinterpret_cast<const double *>(reinterpret_cast<const unsigned char *>(next) + SLOT);
+        nextBar += 8;
+        if (next == reinterpret_cast<const double *>(base + NS * SLOT)) {
+            next = reinterpret_cast<const double *>(base);
+            nextBar -= 8 * NS;
+            nextPar ^= 1;
+        }
+        float *const spare = lcur;
+        lcur = lnext;
+        lnext = spare;
+        planeOk = !__syncthreads_or(!ok);
+        stop = stopAt[t & 1] != 0;
+        if (tid == 0 && !stop && t + NS < nseq) {  // every reader of plane c - 1 = t has passed the barrier
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue(t + NS);
+        }
+        t++;
+        return t < nplanes && !stop;
+    };
+    int plain = 0;  // plain planes to do next
+
+    // step t: plane c = t + 1 from planes m, c, p; false when the loop ends or plain planes are next
     auto step = [&](Own &m, Own &c, Own &p) -> bool {
         if (__builtin_expect(!planeOk, 0)) {  // move the range to the values of planes c - 1 and c (uniform)
             unsigned top = 0;
+            // (written after the barriers below)
+            const int in = t == missAt + 1 ? missed + 1 : 1, n = in > 1 ? nextPlain : PLAIN;
             for (int q = t; q <= t + 1; q++) {
                 const uint2 *w = reinterpret_cast<const uint2 *>(slotOf(q));
 #pragma unroll
@@ -241,6 +323,14 @@ __global__ void __launch_bounds__(TX *TY, MINB)
                 E = e;
                 splitOwn(slotOf(t), m);
                 planeOk = !__syncthreads_or(!splitPlane(slotOf(t + 1), lcur, c));
+            }
+            if (!planeOk) {
+                if (tid == 0) {
+                    missAt = t, missed = in;
+                    nextPlain = in < MISSES ? n : n < PLAIN_MAX ? 2 * n : n;
+                }
+                plain = in >= MISSES ? n : 1;
+                return false;
             }
         }
         await(nextBar, nextPar, t);
@@ -302,8 +392,8 @@ __global__ void __launch_bounds__(TX *TY, MINB)
             for (int r = 0; r < JT; r++) mags[r][0] = mags[r][1] = 1.0f;
         }
         if (__builtin_expect(!fast, 0)) {
-            // values outside the range near these cells, or a quotient that is zero (all six neighbours are +0) or
-            // small: on the FP64 unit, from the doubles of the slots
+            // values outside the range in the planes beside this one, or a quotient that is zero (all six neighbours are
+            // +0) or small: on the FP64 unit, from the doubles of the slots
             const double *pm = slotOf(t) + own, *pc = slotOf(t + 1) + own, *pp = next + own;
 #pragma unroll
             for (int r = 0; r < JT; r++, pm += BX, pc += BX, pp += BX) {
@@ -322,47 +412,30 @@ __global__ void __launch_bounds__(TX *TY, MINB)
                 }
             }
         }
-#pragma unroll
-        for (int r = 0; r < JT; r++) {
-            double *o = out + r * b.s1;
-            if (__builtin_expect((cells >> 2 * r & 3) == 3, 1)) {
-                st2cs(o, make_double2(v[r][0], v[r][1]));
-                if (U) st2cs(o + toOut2, make_double2(v[r][0], v[r][1]));  // A = B into A's second buffer
-            } else {
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    if (cells >> (2 * r + e) & 1) {
-                        o[e] = v[r][e];
-                        if (U) o[toOut2 + e] = v[r][e];
-                    } else if (U && (cells >> (2 * r + e) & 16)) {
-                        o[toOut2 + e] = slotOf(t + 1)[own + r * BX + e];
-                    }
-                }
-            }
-        }
-        out += b.s0;
-        next = reinterpret_cast<const double *>(reinterpret_cast<const unsigned char *>(next) + SLOT);
-        nextBar += 8;
-        if (next == reinterpret_cast<const double *>(base + NS * SLOT)) {
-            next = reinterpret_cast<const double *>(base);
-            nextBar -= 8 * NS;
-            nextPar ^= 1;
-        }
-        float *const spare = lcur;
-        lcur = lnext;
-        lnext = spare;
-        planeOk = !__syncthreads_or(!nextOk);
-        stop = stopAt[t & 1] != 0;
-        if (tid == 0 && !stop && t + NS < nseq) {  // every reader of plane c - 1 = t has passed the barrier
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            issue(t + NS);
-        }
-        t++;
-        return t < nplanes && !stop;
+        store(v);
+        return advance(nextOk);
     };
     // three steps a trip, so that the limbs stay where they are
     if (!stop && nplanes > 0)
-        while (step(oa, ob, oc) && step(ob, oc, oa) && step(oc, oa, ob)) {
+        while (true) {
+            while (step(oa, ob, oc) && step(ob, oc, oa) && step(oc, oa, ob)) {
+            }
+            if (plain == 0) break;
+            bool more = true;
+            for (; plain > 0 && more; plain--) {
+                await(nextBar, nextPar, t);
+                if (cells & MINE) {
+                    double v[JT][2];
+                    native(v);
+                    store(v);
+                }
+                more = advance(true);
+            }
+            if (!more) break;
+            plain = 0;
+            if (tid == 0) missAt = t - 1;
+            splitOwn(slotOf(t), oa);
+            planeOk = !__syncthreads_or(!splitPlane(slotOf(t + 1), lcur, ob));
         }
     if (U) {
         flushMax();
