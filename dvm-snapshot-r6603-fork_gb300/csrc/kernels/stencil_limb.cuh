@@ -450,20 +450,23 @@ __global__ void __launch_bounds__(TX *TY, MINB)
 
 // The grid of kStencil3L with JT rows per thread and `ctas` CTAs resident per SM: the number of chunks of planes that
 // costs least, a chunk of n planes taking about n + 4 steps (the first copies' latency and two planes split ahead),
-// rounds of CTAs one after the other.
+// rounds of CTAs one after the other.  Of the counts that take the same rounds the largest costs least, so the rounds
+// are gone through, not the counts: those took the host 130 us a call for a box of 60000 planes of 8 x 32.
 St3Geom stLGeom(const long lo[3], const long hi[3], int jt, int ctas) {
     St3Geom g{};
     g.ok = hi[0] >= lo[0] && hi[1] >= lo[1] && hi[2] >= lo[2] && lo[2] >= 0;
     if (!g.ok) return g;
     g.p0 = lo[2] >> 1;
     const long gx = ((hi[2] >> 1) - g.p0 + TX) / TX, gy = (hi[1] - lo[1] + TY * jt) / (TY * jt);
-    const long ni = hi[0] - lo[0] + 1, resident = (long)smCount() * ctas;
-    long best = ni, bestCost = -1;
-    for (long want = 1; want <= ni && want <= 65535; want++) {
-        const long n = (ni + want - 1) / want, chunks = (ni + n - 1) / n;
-        const long cost = (gx * gy * chunks + resident - 1) / resident * (n + 4);
-        if (bestCost < 0 || cost < bestCost) bestCost = cost, best = n;
-        if (gx * gy * chunks > 64 * resident) break;  // further chunks only add their first planes
+    const long ni = hi[0] - lo[0] + 1, resident = (long)smCount() * ctas, tiles = gx * gy;
+    const long most = ni < 65535 ? ni : 65535;  // chunks
+    const long first = (tiles + resident - 1) / resident;
+    long best = ni, bestCost = first * (ni + 4);
+    // (64 rounds more: further chunks only add their first planes)
+    for (long rounds = first; rounds * 5 < bestCost && rounds <= first + 64; rounds++) {
+        const long fit = rounds * resident / tiles, n = (ni + (fit < most ? fit : most) - 1) / (fit < most ? fit : most);
+        const long cost = (tiles * ((ni + n - 1) / n) + resident - 1) / resident * (n + 4);
+        if (cost < bestCost) bestCost = cost, best = n;
     }
     g.ichunk = (int)best;
     const long gz = (ni + best - 1) / best;
