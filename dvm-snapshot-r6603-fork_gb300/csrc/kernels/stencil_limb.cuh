@@ -243,16 +243,24 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     // plane t + 1 on the FP64 unit, from the doubles of the slots
     auto native = [&](double v[JT][2]) {
         const double *pm = slotOf(t) + own, *pc = slotOf(t + 1) + own, *pp = next + own;
+        double2 ac[JT];
+        // |B - A| of a cell after the next cell's sum, so that a division runs beside those additions (the pass at 512^3 with
+        // values in [-1, 1) 1937 -> 1924 us, at 600 x 90 x 600 558 -> 549)
+        auto diff = [&](int q) {
+            const double d = sf::nadd(v[q >> 1][q & 1], -(q & 1 ? ac[q >> 1].y : ac[q >> 1].x));
+            if (cells >> q & 1) mb = sf::absmax_bits(d, mb);
+        };
 #pragma unroll
-        for (int r = 0; r < JT; r++, pm += BX, pc += BX, pp += BX) {
-            const double2 ac = *reinterpret_cast<const double2 *>(pc);
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const double first = sf::nadd(sf::nadd(pm[e], pc[e - BX]), e ? ac.x : pc[-1]);
-                v[r][e] = sf::div3p2(sf::nadd(sf::nadd(sf::nadd(first, e ? pc[2] : ac.y), pc[e + BX]), pp[e]), 1);
-                if (U && (cells >> (2 * r + e) & 1)) mb = sf::absmax_bits(sf::nadd(v[r][e], -(e ? ac.y : ac.x)), mb);
-            }
+        for (int q = 0; q < 2 * JT; q++) {
+            const int r = q >> 1, e = q & 1;
+            if (e == 0) ac[r] = *reinterpret_cast<const double2 *>(pc + r * BX);
+            const double first = sf::nadd(sf::nadd(pm[r * BX + e], pc[(r - 1) * BX + e]), e ? ac[r].x : pc[r * BX - 1]);
+            const double sum =
+                sf::nadd(sf::nadd(sf::nadd(first, e ? pc[r * BX + 2] : ac[r].y), pc[(r + 1) * BX + e]), pp[r * BX + e]);
+            if (U && q > 0) diff(q - 1);
+            v[r][e] = sf::div3p2(sum, 1);
         }
+        if (U) diff(2 * JT - 1);
     };
     auto store = [&](const double v[JT][2]) {
 #pragma unroll
