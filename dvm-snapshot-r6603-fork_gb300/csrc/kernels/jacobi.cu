@@ -1438,6 +1438,16 @@ long dvmhgb_jac3d_stnupd_items(const long lo[3], const long hi[3], int variant) 
     return (long)g.grid.x * g.grid.y * g.grid.z;
 }
 
+// Two rows a thread make CTAs of 16 rows: of few rows, an odd number of bands of 8, a good part would be empty, and one
+// row a thread (variant 3) is the faster one.  us, variant 4 / 3, values the limbs hold and in [-1, 1): 2000 x 2 x 2000
+// cells 322 / 201, 427 / 212; 60000 x 8 x 32 349 / 223, 592 / 464; 600 x 24 x 600 72 / 66, 186 / 141; 600 x 72 x 600
+// 172 / 178, 467 / 403; 65^3 13.2 / 12.7, 21.4 / 18.9; from eleven bands on the better share wins: 600 x 88 x 600
+// 205 / 221, 559 / 500.
+int dvmhgb_jac3d_stnupd_default(const long lo[3], const long hi[3]) {
+    const long bands = (hi[1] - lo[1] + TY) / TY;
+    return bands <= 9 && bands % 2 ? 3 : 4;
+}
+
 int dvmhgb_jac3d_stnupd(const double *A, double *Aalt, double *B, const long st[3], const long ext[3],
                         const long lo[3], const long hi[3], double *items, int variant, void *stream) {
     if (variant < 0 || variant >= DVMHGB_JAC3D_STNUPD_VARIANTS) return -1;

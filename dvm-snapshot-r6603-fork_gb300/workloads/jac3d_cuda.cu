@@ -24,7 +24,7 @@
 // the pair: the update kernel, then that stencil in place
 #define DEF_FUSED 25
 // a step's stencil with the next step's update in one pass (the pairing the runtime forms across steps)
-#define DEF_STNUPD 4  // 0.673 a step (variant 5: 0.707; the q61 pass these replaced: 1.09)
+// (dvmhgb_jac3d_stnupd_default: 0.673 a step; the q61 pass that the limb kernels replaced: 1.09)
 
 namespace {
 
@@ -222,7 +222,7 @@ extern "C" void loop_jac3d_stnupd_cuda(DvmType refs[2], DvmType A_hdr[], DvmType
     dvmh_loop_cuda_get_config_C(stn, 0, 0, &threads, &stream, 0);
     dvmh_loop_cuda_get_config_C(upd, 0, 0, &threads, &stream, 0);
     const int variant =
-        dvmhgb_loop_variant_desc(upd, DVMHGB_JAC3D_STNUPD_VARIANTS, DEF_STNUPD, variantDesc(4), NDESC);
+        dvmhgb_loop_variant_desc(upd, DVMHGB_JAC3D_STNUPD_VARIANTS, dvmhgb_jac3d_stnupd_default(lo, hi), variantDesc(4), NDESC);
     double eps, *eps_grid = 0;
     dvmh_loop_cuda_register_red_C(upd, 1, (void **)&eps_grid, 0);
     dvmh_loop_red_init_C(upd, 1, &eps, 0);

@@ -91,6 +91,8 @@ long dvmhgb_jac3d_fused_items(const long lo[3], const long hi[3], int native);
  * the stencil queued past the step's end (deferred loops, dvmh_gb.h). */
 #define DVMHGB_JAC3D_STNUPD_VARIANTS 6
 long dvmhgb_jac3d_stnupd_items(const long lo[3], const long hi[3], int variant);
+/* the variant for a box of which nothing else is known */
+int dvmhgb_jac3d_stnupd_default(const long lo[3], const long hi[3]);
 int dvmhgb_jac3d_stnupd(const double *A, double *Aalt, double *B, const long st[3], const long ext[3],
                         const long lo[3], const long hi[3], double *items, int variant, void *stream);
 int dvmhgb_jac3d_fused(double *A, const double *B, double *Bnew, const long st[3], const long ext[3],

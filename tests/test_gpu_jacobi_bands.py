@@ -103,3 +103,18 @@ def test_signed_fields_are_not_slower(rt, n):
     a.copy_(torch.rand_like(a) * 2 - 1)
     cross = fastest(lambda: rt.dvmhgb_jac3d_stnupd(vp(a), vp(alt), vp(b), st, ext, lo, hi, vp(items), 4, sp))
     assert cross < 1.05 * (fp64 + update)
+
+
+@pytest.mark.parametrize("n", [(2000, 4, 2000), (60000, 10, 34), (600, 26, 600), (256, 255, 256)])
+def test_the_default_shape_is_a_fast_one(rt, n):
+    import torch
+    a = 0.5 + 0.25 * torch.rand(*n, generator=torch.Generator(device="cuda").manual_seed(1), dtype=torch.float64, device="cuda")
+    b, alt = torch.zeros_like(a), torch.zeros_like(a)
+    st, ext, lo, hi = L3(n[1] * n[2], n[2], 1), L3(*n), L3(1, 1, 1), L3(*[q - 2 for q in n])
+    sp = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def time(v):
+        items = torch.zeros(rt.dvmhgb_jac3d_stnupd_items(lo, hi, v), dtype=torch.float64, device="cuda")
+        return fastest(lambda: rt.dvmhgb_jac3d_stnupd(vp(a), vp(alt), vp(b), st, ext, lo, hi, vp(items), v, sp))
+
+    assert time(rt.dvmhgb_jac3d_stnupd_default(lo, hi)) < 1.15 * min(time(v) for v in (0, 1, 2, 3, 4))

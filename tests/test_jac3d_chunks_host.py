@@ -46,3 +46,8 @@ def test_many_planes_do_not_cost_host_time(rt):
     for _ in range(200):
         rt.dvmhgb_jac3d_stnupd_items(lo, hi, 4)
     assert (time.perf_counter() - t) / 200 < 20e-6  # 1 us; 130 when every count was looked at
+
+
+@pytest.mark.parametrize("rows,variant", [(1, 3), (8, 3), (9, 4), (16, 4), (17, 3), (65, 3), (72, 3), (73, 4), (81, 4), (510, 4)])
+def test_few_rows_take_one_a_thread(rt, rows, variant):
+    assert rt.dvmhgb_jac3d_stnupd_default(L3(1, 3, 1), L3(500, 2 + rows, 70)) == variant
