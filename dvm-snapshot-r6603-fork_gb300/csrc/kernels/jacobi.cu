@@ -1052,33 +1052,43 @@ struct Slabs {
     int n;
     long lo[6][3], cnt[6][3];  // axes outermost first; axes the array does not have: 0 and 1
     long start[7];             // threads before the slab, a multiple of 32
-    int wide[6];               // a warp per row (else a thread per row)
+    long pieces[6];            // pieces of a row, one warp each (0: a thread per row)
     long st[3];
 };
+constexpr long PIECE = 1024;
+// a / b for a >= 0, b > 0; a 64-bit division takes about three times the instructions of a 32-bit one
+__device__ __forceinline__ long quotient(long a, long b) { return (a | b) >> 32 ? a / b : (long)((unsigned)a / (unsigned)b); }
 
-// One row (fixed outer indices) per warp where rows have at least 32 elements, one per thread where they are shorter
-// (the faces across the innermost axis: one element each).  Bound by latency: 1.6 M elements around a 512^3 box take
-// 5 us; a thread per element with its three 64-bit divisions took 41.
-__global__ void __launch_bounds__(256) kCopyOutside(const double *__restrict__ src, double *__restrict__ dst, Slabs s) {
+// Rows (fixed outer indices) of at least 32 elements in pieces of up to 1024, one per warp; a shorter row per thread (the
+// faces across the innermost axis: one element each).  Bound by latency: 1.6 M elements around a 512^3 box take 5 us; a
+// thread per element with its three 64-bit divisions took 41.  A whole row per warp is slow where rows are long and few:
+// 20 M elements around a box of rank 1 took 248 ms (a thread per element: 121 us, now 54), 4 rows of 5 M 61 ms (71 us, now
+// 28).  40 registers a thread, six CTAs an SM: at 80, 2000 x 2000 x 3 cells took 97 us in place of 85.
+__global__ void __launch_bounds__(256, 6) kCopyOutside(const double *__restrict__ src, double *__restrict__ dst, Slabs s) {
     gbdev::nextMayLaunch();
     for (long t = blockIdx.x * 256L + threadIdx.x; t < s.start[s.n]; t += gridDim.x * 256L) {
         int q = 0;
         while (t >= s.start[q + 1]) q++;
         const long u = t - s.start[q];
-        const long row = s.wide[q] ? u >> 5 : u;
+        const long pieces = s.pieces[q];
+        const long row = pieces > 1 ? quotient(u >> 5, pieces) : pieces ? u >> 5 : u;
         if (row >= s.cnt[q][0] * s.cnt[q][1]) continue;
-        const long c0 = row / s.cnt[q][1], c1 = row - c0 * s.cnt[q][1];
-        const long off = (s.lo[q][0] + c0) * s.st[0] + (s.lo[q][1] + c1) * s.st[1] + s.lo[q][2] * s.st[2];
-        const long step = s.wide[q] ? 32 : 1, n = s.cnt[q][2];
-        long c = s.wide[q] ? u & 31 : 0;
-        for (; c + 7 * step < n; c += 8 * step) {
+        const long c0 = quotient(row, s.cnt[q][1]), c1 = row - c0 * s.cnt[q][1];
+        // this thread's elements of the row: `left` of them, `step` apart
+        const long first = pieces ? ((u >> 5) - row * pieces) * PIECE + (u & 31) : 0, n = s.cnt[q][2];
+        const long off = (s.lo[q][0] + c0) * s.st[0] + (s.lo[q][1] + c1) * s.st[1] + (s.lo[q][2] + first) * s.st[2];
+        const long step = pieces ? 32 * s.st[2] : s.st[2];
+        int left = (int)(pieces ? (min(n - first, PIECE - (u & 31)) + 31) >> 5 : n);
+        const double *from = src + off;
+        double *to = dst + off;
+        for (; left >= 8; left -= 8, from += 8 * step, to += 8 * step) {
             double v[8];
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = src[off + (c + e * step) * s.st[2]];
+            for (int e = 0; e < 8; e++) v[e] = from[e * step];
 #pragma unroll
-            for (int e = 0; e < 8; e++) dst[off + (c + e * step) * s.st[2]] = v[e];
+            for (int e = 0; e < 8; e++) to[e * step] = v[e];
         }
-        for (; c < n; c += step) dst[off + c * s.st[2]] = src[off + c * s.st[2]];
+        for (; left > 0; left--, from += step, to += step) *to = *from;
     }
     gbdev::waitForKernelBefore();  // launched beside another kernel: ends after it
 }
@@ -1107,9 +1117,9 @@ int copyOutside(int rank, const double *src, double *dst, const long *st, const 
                 empty = empty || h < l;
             }
             if (empty) continue;
-            s.wide[q] = s.cnt[q][2] >= 32;
+            s.pieces[q] = s.cnt[q][2] >= 32 ? (s.cnt[q][2] + PIECE - 1) / PIECE : 0;
             const long rows = s.cnt[q][0] * s.cnt[q][1];
-            s.start[q + 1] = s.start[q] + (s.wide[q] ? rows * 32 : (rows + 31) / 32 * 32);
+            s.start[q + 1] = s.start[q] + (s.pieces[q] ? rows * s.pieces[q] * 32 : (rows + 31) / 32 * 32);
             s.n++;
         }
     if (s.n == 0) return 0;
