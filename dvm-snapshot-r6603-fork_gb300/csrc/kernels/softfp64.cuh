@@ -372,6 +372,16 @@ SF_HD uint64_t q64(double x, bool &ok, int E = Q64_E) {
     return in ? ((X & MANT) | HID) << e : 0;
 }
 
+// the bits of RN(q 2^(E - 1075)): a difference of q64 values of the range E, E > 53, as a double
+SF_HD uint64_t fixed64(uint64_t q, int E) {
+    if (q == 0) return 0;
+    const int z = clz64(q);
+    const uint64_t n = q << z, m = n >> 11;  // the leading one at bit 63, 11 bits to round away
+    const uint32_t rest = (uint32_t)n & 0x7FF;
+    // (the significand's leading one adds 1 to the exponent field, a carry out of it 2)
+    return ((uint64_t)(uint32_t)(E + 10 - z) << 52) + m + (uint64_t)((rest > 0x400) | ((rest == 0x400) & (uint32_t)(m & 1)));
+}
+
 // ---------------------------------------------------------------- 61-bit fixed point (stencil sums)
 //
 // A double x = +0 or 2^-9 <= x < 1 is an integer multiple of 2^-61 below 2^61
