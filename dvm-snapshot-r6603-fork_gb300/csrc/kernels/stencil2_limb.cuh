@@ -9,8 +9,12 @@
 // the heat kernel does (rowlimb.cuh).  Rows i-1, i, i+1 are in registers as limbs,
 // the next seven on their way to shared memory; the left and right neighbours come
 // by shuffles.  The range of the limbs follows the values of the warp's rows; a row
-// that does not fit it is computed on the FP64 unit.  |B - A| is taken on the FP64
-// unit, which is otherwise idle: one operation a cell, used a row later.
+// that does not fit it is computed on the FP64 unit; after a move in vain the next
+// 32 such rows are not tried (values of 24 decades at 4097^2, a move in every row:
+// stencil 172 us, fused 341; with every sum on the FP64 unit 169 and 259; now 138 and
+// 245).
+// |B - A| is taken on the FP64 unit, which is otherwise idle: one operation a cell,
+// used a row later.
 //
 // What bounds it: instruction issue, about 200 (FUSED 330) a row of a chunk, at 16
 // warps an SM.  With one row in flight in registers in place of the ring the
@@ -150,17 +154,24 @@ __global__ void __launch_bounds__(256, 2)
         double *out = Out + i0 * s0 + j, *a = FUSED ? A + i0 * s0 + j : nullptr;
         long i = i0;
         int left = count;
+        int hold = 0;  // rows that are not tried in another range, the last move having been in vain
+        constexpr int HOLD = 32;
 
         // row i from up, mid, dn; up then takes row i + 2's place
         auto step = [&](rows::Row &up, rows::Row &mid, rows::Row &dn) -> bool {
             const bool more = left > 1;
             if (__builtin_expect(!(up.ok && mid.ok && dn.ok), 0)) {
-                const int e = rows::rangeOf(up, mid, dn, E);
-                if (e != E) {  // move the range
-                    E = e;
-                    again(i - 1, up);
-                    again(i, mid);
-                    again(i + 1, dn);
+                if (hold > 0) {
+                    hold--;
+                } else {
+                    const int e = rows::rangeOf(up, mid, dn, E);
+                    if (e != E) {  // move the range
+                        E = e;
+                        again(i - 1, up);
+                        again(i, mid);
+                        again(i + 1, dn);
+                        if (!(up.ok && mid.ok && dn.ok)) hold = HOLD;
+                    }
                 }
             }
             double v0, v1;
