@@ -650,10 +650,16 @@ __device__ __forceinline__ unsigned long long hypPack(long a, long b, long c) {
 // over the columns in closed form) and its tiles in the order (c, then a).
 // Thread u takes the diagonal s = a + b = smax - u of the plane (c = d - s:
 // ascending with u), counts its tiles, and writes them, a ascending, at its
-// place in the CTA's scan.
+// place in the CTA's scan.  It clears the tiles' flags too when they are given; and does nothing where the sweep that
+// takes the list hands out none of it.
+constexpr unsigned NO_HAND_OUT = 1u << 30;  // a counter from which no tile or column is handed out: there are fewer
 template <int G>
-__global__ void __launch_bounds__(256) kHypTable(HGeo g, unsigned long long *table) {
+__global__ void __launch_bounds__(256) kHypTable(HGeo g, unsigned long long *table, const unsigned *counter,
+                                                 int *flags) {
     __shared__ long long part[8];
+    if (*counter >= NO_HAND_OUT) return;
+    if (flags)
+        for (long q = blockIdx.x * 256L + threadIdx.x; q < g.na * g.nb * g.ncg; q += gridDim.x * 256L) flags[q] = 0;
     const long d = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     long long before = 0;
@@ -922,7 +928,7 @@ __global__ void __launch_bounds__(NT) kSorHyp(double *A, HGeo g, const double *w
     }
 }
 
-// ---- columns of hyperplane tiles (variant 5, the default)
+// ---- columns of hyperplane tiles (variant 5)
 //
 // A CTA of WI = 4 warps walks a column (a, b) of 16 x 8 rows from its first tile to its last, its warps in lockstep (a
 // barrier per step).  What one tile leaves to the next stays in the CTA: the rows' last new values, the squares of an
@@ -940,8 +946,9 @@ __global__ void __launch_bounds__(NT) kSorHyp(double *A, HGeo g, const double *w
 // of 740 - 950 (the dependent chain of split, five additions, assembly, two FP64 operations and the barrier), 700 for
 // the faces, 500 to publish, 1,000 until the next column sees it.  Measured per sweep (values in one range), against
 // tiles of one warp (variant 4) and one tile of 16 x 8 rows per CTA and hand-out, with all sums on FP64: 97^3 269 us
-// (366, 316), 384^3 1690 us (2035, 2037).  With signed values: 97^3 300 us (365), 384^3 2175 us (2035): variant 4 remains
-// for large boxes of those.  Storing the last rows in the steps and publishing from another warp than the one that
+// (366, 316), 384^3 1690 us (2035, 2037).  With signed values: 97^3 300 us (365), 384^3 2155 us (2033): there variant 4 is
+// taken (hypChoice).  The squares and trees of the residual on the integer pipe, two FP64 instructions less a step:
+// slower throughout (signed 384^3 2500, 97^3 374; without branches 2770 and 411).  Storing the last rows in the steps and publishing from another warp than the one that
 // polls, instead of a store phase, a barrier and warp 0 for both: 281 -> 269, 1747 -> 1690.  What did not help: limbs
 // kept in shared memory and split once by their producer (unrolled or not, 288 and 1788 us), four CTAs per SM (1946 us
 // at 384^3), 32 x 8 rows (2166 us), 8 x 8 (1749 us; 320 us at 97^3), unrolled steps (instruction cache: 1821 - 1880 us).
@@ -1006,6 +1013,7 @@ __global__ void __launch_bounds__(32 * WI, 12 / WI) kSorHypCol(double *A, HGeo g
     // warps with other things to do neither poll (warp 0 loads the -i face) nor publish and poll at once
     constexpr int POLL = 32 * (WI / 2), PUBLISH = NTc - 1;
     gbdev::nextMayLaunch();
+    gbdev::waitForKernelBefore();
     const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5, li = lane / TJ, lj = lane % TJ;
     const int lr = li, lp = lj;     // staging: a lane copies position lp of rows lr, lr + 4, ...
     double *box = sm + wi * TI * RS;                   // the warp's rows and their faces
@@ -1316,11 +1324,14 @@ HypScratch hypScratch(const HGeo &g) {
 }
 
 // one hyperplane sweep.  cta: columns of CTA_TI x CTA_TJ rows, one per CTA (kSorHypCol); else the tile list, then
-// tiles of 4 x 8 rows, one per warp (kSorHyp)
+// tiles of 4 x 8 rows, one per warp (kSorHyp).  chosen: one of the two sweeps after kSorSample; their counters and the
+// progress words are cleared already.  The columns are launched while that runs where they take every place of the GPU (14
+// us less a sweep at 384^3); fewer would find others than alone, several on an SM (32 columns: 1405 -> 1670 us), and
+// launched beside the columns the list and the tiles' sweep that wait cost more than their launches (250^3: 890 -> 1092)
 constexpr int CTA_TI = 16, CTA_TJ = 8;
 template <int G>
 int sweepHyp(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3], const double *wDev,
-             double *items, void *scratch, int *status, Bound bound, bool cta, cudaStream_t s) {
+             double *items, void *scratch, int *status, Bound bound, bool cta, cudaStream_t s, bool chosen = false) {
     HGeo g;
     if (!hypGeo<G>(st, ext, lo, hi, cta ? CTA_TI : TI, cta ? CTA_TJ : TJ, g)) return -1;
     const HypScratch sc = hypScratch<G>(g);
@@ -1331,19 +1342,25 @@ int sweepHyp(double *A, const long st[3], const long ext[3], const long lo[3], c
         constexpr int WI = CTA_TI / TI;
         using H = HypCol<G, WI>;
         const long ncols = g.na * g.nb;  // a progress word each (of the scratch, sized for one flag per tile)
-        if (cudaMemsetAsync(scratch, 0, sc.flagsOff + sizeof(int) * (size_t)ncols, s) != cudaSuccess) return -1;
+        if (!chosen && cudaMemsetAsync(scratch, 0, sc.flagsOff + sizeof(int) * (size_t)ncols, s) != cudaSuccess)
+            return -1;
         static std::atomic<int> occCache[gbdev::MAX_DEVICES];
         const int occ = gbdev::residentCtas(occCache, kSorHypCol<G, WI>, H::NTc, H::SMEM);
         long grid = (long)occ * gbdev::smCount();  // all CTAs resident at once: waits always resolve
         if (grid > ncols) grid = ncols;
-        kSorHypCol<G, WI><<<(unsigned)grid, H::NTc, H::SMEM, s>>>(A, g, wDev, flags, counter, items, status, bound);
+        const auto sweep = kSorHypCol<G, WI>;
+        if (!chosen || grid == ncols)
+            sweep<<<(unsigned)grid, H::NTc, H::SMEM, s>>>(A, g, wDev, flags, counter, items, status, bound);
+        else if (gbdev::launchAfterShared(sweep, (unsigned)grid, H::NTc, H::SMEM, s, A, g, wDev, flags, counter, items,
+                                          status, bound) != cudaSuccess)
+            return -1;
         dvmhgb_count_launches(1);
     } else {
         using H = Hyp<G>;
         unsigned long long *table = (unsigned long long *)(base + sc.tableOff);
         double *carry = (double *)(base + sc.carryOff);
-        if (cudaMemsetAsync(scratch, 0, sc.tableOff, s) != cudaSuccess) return -1;
-        kHypTable<G><<<(unsigned)g.nlev, 256, 0, s>>>(g, table);
+        if (!chosen && cudaMemsetAsync(scratch, 0, sc.tableOff, s) != cudaSuccess) return -1;
+        kHypTable<G><<<(unsigned)g.nlev, 256, 0, s>>>(g, table, counter, chosen ? flags : nullptr);
         static std::atomic<int> occCache[gbdev::MAX_DEVICES];
         const int occ = gbdev::residentCtas(occCache, kSorHyp<G>, NT, H::SMEM);
         long grid = (long)occ * gbdev::smCount();
@@ -1354,6 +1371,91 @@ int sweepHyp(double *A, const long st[3], const long ext[3], const long lo[3], c
         dvmhgb_count_launches(2);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// Columns (variant 5) or tiles one by one (variant 4).  A sweep goes through the planes a + b + c of its tiles, those of
+// the columns fewer (16 rows along i in place of 4) and slower, the more so the more of its tiles sum on the FP64 unit and
+// the more columns there are.  Measured, us a sweep as a graph, columns / tiles, values in one range and in [-1, 1):
+//   up to a column an SM      97^3 282 / 364, 302 / 366; 60 x 60 x 2000 1394 / 1429, 1521 / 1432; 18 x 200 x 300 469 / 461,
+//                             496 / 462; 100 x 100 x 1000 886 / 979, 948 / 979
+//   up to two                 160^3 520 / 618, 599 / 620; 190^3 644 / 749, 767 / 748; 40 x 500 x 400 1059 / 974, 1211 / 974;
+//                             500 x 40 x 400 878 / 1259, 978 / 1260; 60 x 400 x 200 781 / 754, 895 / 752
+//   more                      200^3 740 / 798, 902 / 802; 230^3 875 / 955, 1146 / 957; 300^3 1198 / 1379, 1517 / 1379; 384^3
+//                             1729 / 2033, 2224 / 2033; 400 x 400 x 40 1066 / 1311, 1277 / 1311
+// So a plane of columns costs 2 .. 10, 12 .. 32 and 18 .. 50 percent more than one of tiles.  With up to two columns an SM
+// the middle decides.  With more, samples of the field do: `limit` is the number of those that the limbs do not hold up
+// to which the columns are taken, three quarters of what a straight line between the two fields gives, since half of
+// the tiles on the FP64 unit (a wave about zero) cost more than half the difference (230^3 1059, 300^3 1417, 384^3 1958).
+constexpr int SAMPLES = 512, SAMPLE_THREADS = 128;
+int hypChoice(const long lo[3], const long hi[3], unsigned &limit) {
+    HGeo t, c;
+    if (!hypGeo<8>(nullptr, nullptr, lo, hi, CTA_TI, CTA_TJ, c) || !hypGeo<8>(nullptr, nullptr, lo, hi, TI, TJ, t))
+        return 5;
+    const long cols = c.na * c.nb, sms = gbdev::smCount(), tiles = 100 * t.nlev;
+    if (cols <= 2 * sms) return (cols <= sms ? 106 : 122) * c.nlev < tiles ? 5 : 4;
+    const long in = 118 * c.nlev, out = 150 * c.nlev;
+    if (out <= tiles) return 5;
+    if (in >= tiles) return 4;
+    limit = (unsigned)(SAMPLES * 3 / 4 * (tiles - in) / (out - in));
+    return DVMHGB_SOR3D_BY_FIELD;
+}
+
+// A sample is 4 x 8 rows of 64 cells, what a warp of the columns decides by: negative values among them, or several that
+// are eight binades below the largest, and its sums take the FP64 unit.  The last CTA to end stops the hand-out of the
+// sweep that those do not favour; state: samples that the limbs do not hold, CTAs that have ended.  About 3 us.
+__global__ void __launch_bounds__(SAMPLE_THREADS) kSorSample(const double *__restrict__ A, HGeo g, unsigned *state,
+                                                             unsigned limit, unsigned *columns, unsigned *tiles) {
+    gbdev::nextMayLaunch();
+    const int lane = threadIdx.x & 31;
+    const unsigned q = blockIdx.x * (SAMPLE_THREADS / 32) + (threadIdx.x >> 5) + 1;
+    // spread over the box by the multiples of three irrational numbers (1/x, 1/x^2, 1/x^3 for x^4 = x + 1)
+    const long ni = g.hi0 - g.lo0 + 1;
+    const long i0 = (long)((unsigned long long)(q * 0xD1B54A33u) * (unsigned long long)ni >> 32);
+    const long j0 = (long)((unsigned long long)(q * 0xABC98389u) * (unsigned long long)g.nj >> 32);
+    const long k0 = (long)((unsigned long long)(q * 0x8CB92BA7u) * (unsigned long long)g.nk >> 32);
+    unsigned most = 0, h[64];  // high words of two cells of each row, all on their way at once
+#pragma unroll
+    for (int u = 0; u < 64; u++) {
+        const long i = i0 + u / 16, j = j0 + u / 2 % 8, k = k0 + u % 2 * 32 + lane;
+        h[u] = i < ni && j < g.nj && k < g.nk
+                   ? sf::hi32(sf::bits(__ldg(A + (g.lo0 + i) * g.s0 + (g.lo1 + j) * g.s1 + g.lo2 + k)))
+                   : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < 64; u++) most = max(most, h[u]);
+    most = __reduce_max_sync(0xffffffffu, most);
+    const unsigned low = most >> 20 > 8u ? ((most >> 20) - 8u) << 20 : 0u;
+    int small = 0;
+#pragma unroll
+    for (int u = 0; u < 64; u++) small += h[u] && h[u] < low;
+    small = __reduce_add_sync(0xffffffffu, small);
+    if (lane == 0 && (most >> 31 || small >= 8)) atomicAdd(state, 1u);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(state + 1, 1u) == gridDim.x - 1) *(atomicAdd(state, 0u) > limit ? columns : tiles) = NO_HAND_OUT;
+    }
+}
+
+// scratch of the sweep that the field chooses: the columns' (counter and, in its line, kSorSample's state; progress
+// words), then the tiles'
+size_t columnsBytes(const long lo[3], const long hi[3]) {
+    const size_t cols = (size_t)(((hi[0] - lo[0]) / CTA_TI + 1) * ((hi[1] - lo[1]) / CTA_TJ + 1));
+    return (256 + sizeof(int) * cols + 255) / 256 * 256;
+}
+
+int sweepByField(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3], const double *wDev,
+                 double *items, void *scratch, int *status, Bound bound, unsigned limit, cudaStream_t s) {
+    HGeo g;
+    if (!hypGeo<8>(st, ext, lo, hi, TI, TJ, g)) return -1;
+    const size_t cols = columnsBytes(lo, hi);
+    unsigned *columns = (unsigned *)scratch, *tiles = (unsigned *)((char *)scratch + cols);
+    // (the tiles' counter too; their flags are kHypTable's)
+    if (cudaMemsetAsync(scratch, 0, cols + hypScratch<8>(g).flagsOff, s) != cudaSuccess) return -1;
+    kSorSample<<<SAMPLES / (SAMPLE_THREADS / 32), SAMPLE_THREADS, 0, s>>>(A, g, columns + 32, limit, columns, tiles);
+    dvmhgb_count_launches(1);
+    if (sweepHyp<8>(A, st, ext, lo, hi, wDev, items, columns, status, bound, true, s, true) != 0) return -1;
+    return sweepHyp<8>(A, st, ext, lo, hi, wDev, items, tiles, status, bound, false, s, true);
 }
 
 }  // namespace
@@ -1395,6 +1497,26 @@ int dvmhgb_sor3d_sweep_bounded(double *A, const long st[3], const long ext[3], c
         case 16: return sweepT<16>(A, g, wDev, items, scratch, status, bound, s);
         default: return sweepT<8>(A, g, wDev, items, scratch, status, bound, s);
     }
+}
+
+int dvmhgb_sor3d_default_variant(const long lo[3], const long hi[3]) {
+    unsigned limit;
+    return hypChoice(lo, hi, limit);
+}
+
+long dvmhgb_sor3d_by_field_scratch_bytes(const long lo[3], const long hi[3]) {
+    const long tiles = dvmhgb_sor3d_scratch_bytes(lo, hi, 4);
+    return tiles < 0 ? -1 : (long)columnsBytes(lo, hi) + tiles;
+}
+
+int dvmhgb_sor3d_sweep_by_field(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3],
+                                const double *wDev, double *items, void *scratch, int *status, void *stream) {
+    Geo g;
+    if (!A || !wDev || !items || !scratch || !status || !geo(st, ext, lo, hi, 8, g)) return -1;
+    const Bound bound{SPIN_LIMIT, 0};
+    unsigned limit = SAMPLES / 2;  // where one is always the faster, either will do
+    hypChoice(lo, hi, limit);
+    return sweepByField(A, st, ext, lo, hi, wDev, items, scratch, status, bound, limit, (cudaStream_t)stream);
 }
 
 int dvmhgb_sor3d_sweep(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3],

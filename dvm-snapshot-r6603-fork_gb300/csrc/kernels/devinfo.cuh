@@ -17,18 +17,24 @@ __device__ __forceinline__ void nextMayLaunch() { asm volatile("griddepcontrol.l
 __device__ __forceinline__ void waitForKernelBefore() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... Params, typename... Args>
-inline cudaError_t launchAfter(void (*kernel)(Params...), unsigned blocks, unsigned threads, cudaStream_t s,
-                               Args... args) {
+inline cudaError_t launchAfterShared(void (*kernel)(Params...), unsigned blocks, unsigned threads, size_t shared,
+                                     cudaStream_t s, Args... args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c{};
     c.gridDim = dim3(blocks);
     c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = shared;
     c.stream = s;
     c.attrs = &attr;
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, kernel, Params(args)...);
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launchAfter(void (*kernel)(Params...), unsigned blocks, unsigned threads, cudaStream_t s,
+                               Args... args) {
+    return launchAfterShared(kernel, blocks, threads, 0, s, args...);
 }
 
 constexpr int MAX_DEVICES = 64;

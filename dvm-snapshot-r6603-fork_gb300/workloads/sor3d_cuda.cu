@@ -12,13 +12,13 @@
 #include "dvmh_gb.h"
 #include "dvmh_gb_kernels.h"
 
-#define SOR_DEFAULT_VARIANT 5
+#define N_VARIANTS (DVMHGB_SOR3D_VARIANTS + 1)  // and the choice by the field
 
 // the variants as the tuner's variant model sees them: family 3 (this program),
 // the tile depth along k (64: streaming columns; hyperplanes per tile for the
 // hyperplane tiles), tile kind (0 box, 1 streaming column, 2 hyperplane tile per
-// warp, 3 column of hyperplane tiles per CTA)
-static const float sorDesc[6 * 3] = {3, 32, 0, 3, 16, 0, 3, 8, 0, 3, 64, 1, 3, 8, 2, 3, 8, 3};
+// warp, 3 column of hyperplane tiles per CTA, 4 one of those two by the field)
+static const float sorDesc[N_VARIANTS * 3] = {3, 32, 0, 3, 16, 0, 3, 8, 0, 3, 64, 1, 3, 8, 2, 3, 8, 3, 3, 8, 4};
 
 extern "C" void loop_sor3d_cuda(DvmType *pLoopRef, DvmType A_hdr[], double *s_ptr, double *w_ptr) {
     (void)s_ptr;
@@ -49,10 +49,16 @@ extern "C" void loop_sor3d_cuda(DvmType *pLoopRef, DvmType A_hdr[], double *s_pt
     dvmh_loop_cuda_register_red_C(loop_ref, 1, (void **)&s_grid, 0);
     dvmh_loop_red_init_C(loop_ref, 1, &s, 0);
     // tile shape: chosen by the runtime's variant tuner
-    const int variant = dvmhgb_loop_variant_desc(loop_ref, DVMHGB_SOR3D_VARIANTS, SOR_DEFAULT_VARIANT, sorDesc, 3);
-    dvmh_loop_cuda_red_prepare_C(loop_ref, 1, dvmhgb_sor3d_items(lo, hi, variant), 0);
-    void *scratch = dvmhgb_loop_scratch(loop_ref, dvmhgb_sor3d_scratch_bytes(lo, hi, variant));
-    if (dvmhgb_sor3d_sweep(A, st, ext, lo, hi, w_dev, s_grid, scratch, dvmhgb_status_word(), variant, stream) != 0) {
+    const int variant =
+        dvmhgb_loop_variant_desc(loop_ref, N_VARIANTS, dvmhgb_sor3d_default_variant(lo, hi), sorDesc, 3);
+    const bool byField = variant == DVMHGB_SOR3D_BY_FIELD;
+    dvmh_loop_cuda_red_prepare_C(loop_ref, 1, dvmhgb_sor3d_items(lo, hi, byField ? 5 : variant), 0);
+    void *scratch = dvmhgb_loop_scratch(loop_ref, byField ? dvmhgb_sor3d_by_field_scratch_bytes(lo, hi)
+                                                          : dvmhgb_sor3d_scratch_bytes(lo, hi, variant));
+    int *status = dvmhgb_status_word();
+    const int rc = byField ? dvmhgb_sor3d_sweep_by_field(A, st, ext, lo, hi, w_dev, s_grid, scratch, status, stream)
+                           : dvmhgb_sor3d_sweep(A, st, ext, lo, hi, w_dev, s_grid, scratch, status, variant, stream);
+    if (rc != 0) {
         fprintf(stderr, "loop_sor3d_cuda: kernel launch rejected its arguments\n");
         exit(1);
     }

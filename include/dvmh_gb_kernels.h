@@ -129,6 +129,16 @@ long dvmhgb_sor3d_items(const long lo[3], const long hi[3], int variant);
 long dvmhgb_sor3d_scratch_bytes(const long lo[3], const long hi[3], int variant);
 int dvmhgb_sor3d_sweep(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3],
                        const double *wDev, double *items, void *scratch, int *status, int variant, void *stream);
+/* The variant for a box of which nothing else is known: 4, 5, or
+ * DVMHGB_SOR3D_BY_FIELD where the faster of the two depends on the values
+ * (columns sum on FP32 limbs what lies in nine binades of positive values).
+ * Then dvmhgb_sor3d_sweep_by_field samples the field and one of the two does
+ * the sweep; items as for variant 5, scratch of its own size. */
+#define DVMHGB_SOR3D_BY_FIELD DVMHGB_SOR3D_VARIANTS
+int dvmhgb_sor3d_default_variant(const long lo[3], const long hi[3]);
+long dvmhgb_sor3d_by_field_scratch_bytes(const long lo[3], const long hi[3]);
+int dvmhgb_sor3d_sweep_by_field(double *A, const long st[3], const long ext[3], const long lo[3], const long hi[3],
+                                const double *wDev, double *items, void *scratch, int *status, void *stream);
 /* The same sweep with its bounded waits made explicit.  Every wait for a
  * predecessor tile (column, variants 3 and 5) polls at most pollLimit times
  * (dvmhgb_sor3d_sweep: 2^24, about 1-4 s) before the kernel writes its timeout
