@@ -1147,7 +1147,7 @@ int copyOutside(int rank, const double *src, double *dst, const long *st, const 
 // row per thread, registers capped for three / four CTAs per SM; v = 14..21:
 // the q61 fixed-point stencil (kStencil3Q) with (CTAs per SM, native CTAs of
 // every den): 14 (4, 0 of 1), 15 (3, 0 of 1), 16 (4, 1 of 2), 17 (4, 1 of 3),
-// 18 (4, 2 of 5), 19 (3, 1 of 2), 20 (4, 1 of 4), 21 (4, 3 of 5); v = 22, 23:
+// 18 (4, 2 of 5), 19 (3, 1 of 2), 20 (4, 1 of 4), 21 (4, 3 of 5); v = 22..26:
 // the stencil on FP32 limbs with its planes staged by TMA (kStencil3L), shapes
 // DVMHGB_LIMB_SHAPES (the fused entry point runs the update and then the stencil
 // into the second buffer for v = 14..26)
@@ -1209,11 +1209,12 @@ int launchSU(const double *A, double *B, double *Aalt, const Box3 &b, const long
 
 // (rows per thread, plane slots, CTAs per SM) of the limb kernels' variants: the stencil's 22 + v (v < 5) and the
 // cross-step pass's v.  At 512^3, us (stencil a call / a batched step of the cross-step pass with the faces' copy beside
-// it and the fold): 0: 703 / 830, 1: 620 / 722, 2: 617 / 686, 3 and 5: 612 / 707, 4: 616 / 673 (six slots 678, seven
-// 706, four 746; three rows a thread at one CTA 873).  Two rows a thread take a quarter fewer instructions per cell and
+// it and the fold): 0: 703 / 830, 1: 620 / 722, 2: 617 / 686, 3: 612 / 707, 4: 616 / 673, 5: - / 678 (seven
+// slots 706, four 746; three rows a thread at one CTA 873).  Two rows a thread take a quarter fewer instructions per cell and
 // hold half the warps: the faster ones where the pass also takes |B - A| and writes twice, and with registers left on
 // the SM for the copy's CTAs; 256^3: 116 against 121, 130^3: 40 against 41.5.
-#define DVMHGB_LIMB_SHAPES(C) C(0, 1, 5, 4) C(1, 1, 5, 3) C(2, 2, 5, 2) C(3, 1, 6, 3) C(4, 2, 8, 2) C(5, 1, 6, 3)
+#define DVMHGB_LIMB_STENCILS(C) C(0, 1, 5, 4) C(1, 1, 5, 3) C(2, 2, 5, 2) C(3, 1, 6, 3) C(4, 2, 8, 2)
+#define DVMHGB_LIMB_SHAPES(C) DVMHGB_LIMB_STENCILS(C) C(5, 2, 6, 2)
 
 template <bool FUSED>
 void launch3(int variant, const St3Geom &g, double *A, const double *B, double *Out, const Box3 &b, double *items,
@@ -1287,7 +1288,7 @@ int dvmhgb_jac3d_stencil(const double *A, double *B, const long st[3], const lon
         int rc = -1;
         switch (native - V3T) {
 #define C(V, JT, NS, MINB) case V: rc = launchT<JT, NS, MINB>(A, B, b, st, lo, hi, (cudaStream_t)stream); break;
-            DVMHGB_LIMB_SHAPES(C)
+            DVMHGB_LIMB_STENCILS(C)
 #undef C
         }
         if (rc != 0) return -1;

@@ -39,7 +39,7 @@ constexpr int NDESC = 8;
 constexpr int V_Q = 14, V_T = 22;  // first fixed-point stencil variant, first TMA-staged one
 // the limb kernels' shapes: rows per thread, planes in the ring, CTAs per SM
 void limbDesc(int shape, float *d) {
-    static const int c[6][3] = {{1, 5, 4}, {1, 5, 3}, {2, 5, 2}, {1, 6, 3}, {2, 8, 2}, {1, 6, 3}};
+    static const int c[6][3] = {{1, 5, 4}, {1, 5, 3}, {2, 5, 2}, {1, 6, 3}, {2, 8, 2}, {2, 6, 2}};
     d[2] = 2.0f + (float)c[shape][1] / 6.0f, d[3] = 0, d[4] = (float)c[shape][0], d[5] = (float)c[shape][2], d[6] = 0;
 }
 void stencilDesc(int v, float *d) {

@@ -86,7 +86,7 @@ long dvmhgb_jac3d_fused_items(const long lo[3], const long hi[3], int native);
  * partials into items (dvmhgb_jac3d_stnupd_items).  24 bytes a cell.  The
  * limb stencil (variant 25 above) with the update on its new values; variants
  * (rows per thread, planes in the ring, CTAs per SM): 0 (1, 5, 4), 1 (1, 5, 3),
- * 2 (2, 5, 2), 3 and 5 (1, 6, 3), 4 (2, 8, 2).
+ * 2 (2, 5, 2), 3 (1, 6, 3), 4 (2, 8, 2), 5 (2, 6, 2).
  * The runtime pairs the loops so when a program's time steps leave
  * the stencil queued past the step's end (deferred loops, dvmh_gb.h). */
 #define DVMHGB_JAC3D_STNUPD_VARIANTS 6
