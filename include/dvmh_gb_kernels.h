@@ -186,6 +186,7 @@ int dvmhgb_heat_many(const dvmhgb_heat_desc *dDev, int n, long totalStrips, void
  * arguments).  dvmhgb_heat_desc_rows sets a descriptor's rows per strip (and its
  * strip count); -1 for sr < 1. */
 #define DVMHGB_HEAT_VARIANTS 10
+#define DVMHGB_HEAT_DEFAULT 2 /* where the loops are not known (a constant: see dvmhgb_heat_default_variant) */
 #define DVMHGB_HEAT_ROWS(v) (8L << ((v) % 5))
 #define DVMHGB_HEAT_CTAS(v) ((v) < 5 ? 2 : 1)
 int dvmhgb_heat_default_variant(const dvmhgb_heat_desc *d, int n);
