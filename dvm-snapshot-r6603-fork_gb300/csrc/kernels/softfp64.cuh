@@ -190,7 +190,7 @@ SF_HD double mul(double a, double b) {
 SF_HD double div3p2(double x, int k) {
     uint64_t X = bits(x);
     uint64_t ex = (X >> 52) & 0x7FF;
-    if (ex - 1 >= 0x7FE) return ndiv(x, 3.0 * (double)(1ull << k));
+    if (ex - 1 >= 0x7FE) return (X << 1) == 0 ? x : ndiv(x, 3.0 * (double)(1ull << k));
     uint64_t n = ((X & MANT) | HID) << 11;  // in [2^63, 2^64)
     uint64_t q = mulhi(n, 0xAAAAAAAAAAAAAAABull) >> 1;
     uint64_t r = n - 3 * q;

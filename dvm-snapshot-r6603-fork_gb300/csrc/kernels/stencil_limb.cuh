@@ -397,26 +397,33 @@ __global__ void __launch_bounds__(TX *TY, MINB)
             }
         } else {
 #pragma unroll
-            for (int r = 0; r < JT; r++) mags[r][0] = mags[r][1] = 1.0f;
+            for (int r = 0; r < JT; r++) {
+                mags[r][0] = mags[r][1] = 1.0f;
+                if (!U) v[r][0] = v[r][1] = 0.0;
+            }
         }
         if (__builtin_expect(!fast, 0)) {
             // values outside the range in the planes beside this one, or a quotient that is zero (all six neighbours are
-            // +0) or small: on the FP64 unit, from the doubles of the slots
+            // +0) or small: on the FP64 unit, from the doubles of the slots.  Alone the stencil keeps the thread's other
+            // quotients; with the update they are made again, since keeping them costs the common path 1 to 3 percent in
+            // every form tried.  512^3, 2 percent of values among zeros: stencil 1703 -> 791 us (q61 kernels 1203), cross-step
+            // pass 2582 -> 2205 (1572; 1300 where they were kept), 130^3 147 -> 67 (64); only zeros 922 -> 818.
             const double *pm = slotOf(t) + own, *pc = slotOf(t + 1) + own, *pp = next + own;
 #pragma unroll
             for (int r = 0; r < JT; r++, pm += BX, pc += BX, pp += BX) {
                 const double2 ac = *reinterpret_cast<const double2 *>(pc);
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
+                    double d = e ? ac.y : ac.x;  // |B - A| of a zero
                     if (mags[r][e] == 0.0f) {
                         v[r][e] = 0.0;
-                    } else {
+                    } else if (U || mags[r][e] < tiny[r][e]) {
                         const double first = sf::nadd(sf::nadd(pm[e], pc[e - BX]), e ? ac.x : pc[-1]);
                         v[r][e] = sf::div3p2(
                             sf::nadd(sf::nadd(sf::nadd(first, e ? pc[2] : ac.y), pc[e + BX]), pp[e]), 1);
+                        if (U) d = sf::nadd(v[r][e], -d);
                     }
-                    if (U && (cells >> (2 * r + e) & 1))
-                        mb = sf::absmax_bits(sf::nadd(v[r][e], -(e ? ac.y : ac.x)), mb);
+                    if (U && (cells >> (2 * r + e) & 1)) mb = sf::absmax_bits(d, mb);
                 }
             }
         }
