@@ -1402,7 +1402,7 @@ int hypChoice(const long lo[3], const long hi[3], unsigned &limit) {
 
 // A sample is 4 x 8 rows of 64 cells, what a warp of the columns decides by: negative values among them, or several that
 // are eight binades below the largest, and its sums take the FP64 unit.  The last CTA to end stops the hand-out of the
-// sweep that those do not favour; state: samples that the limbs do not hold, CTAs that have ended.  About 3 us.
+// sweep that those do not favour; state: samples that the limbs do not hold, CTAs that have ended.  6 us alone at 384^3.
 __global__ void __launch_bounds__(SAMPLE_THREADS) kSorSample(const double *__restrict__ A, HGeo g, unsigned *state,
                                                              unsigned limit, unsigned *columns, unsigned *tiles) {
     gbdev::nextMayLaunch();
